@@ -29,11 +29,13 @@
 //     pick pass over the chosen node's subtree.
 //   * Walks carry no stack: they follow per-node escape links.
 //   * A persistent form keeps the top levels of the octree in shared memory.
-//   * For sparse search lists, one search per warp (k_search_wide): the lanes
-//     evaluate a tree level of candidates side by side and the sum runs in
-//     the reference's order over the collected candidates.
+//   * One search per warp by sums over bins (k_search_bins, bh_bins.cuh): the
+//     lanes evaluate the children of four nodes side by side, and the crossing
+//     is certified against the rounding of the reference's own order; the few
+//     searches too close to call go to k_search_wide, whose sum runs in the
+//     reference's order over the collected candidates.
+#include "bh_bins.cuh"
 #include "bh_eval.cuh"
-#include "bh_wide.cuh"
 #include "rl_context.cuh"
 #include "rl_math.cuh"
 
@@ -67,6 +69,7 @@ struct SearchArgs {
     uint32_t* err;
     unsigned long long* touched;
     KernelParams kernel;
+    int redo_only;  // packet kernel: only the list entries left at kRedo
 };
 
 // Parameters of the network a warp searches in.
@@ -324,7 +327,7 @@ __device__ __forceinline__ void search_task(const SearchArgs& A, const Hot64& H,
     const NetInfo& N = A.nets[A.seg_net[lo]];
     const WarpNet W{ N.theta, N.scale, N.seed, A.seg_net[lo], N.first };
     const uint64_t idx = A.seg_begin[lo] + (uint64_t)(warp_global - A.seg_warp[lo]) * 32 + lane;
-    const bool active = idx < A.seg_end[lo];
+    const bool active = idx < A.seg_end[lo] && (!A.redo_only || A.target[idx] == kRedo);
     if (N.root_leaf) {
         // a network of one neuron: its only candidate is itself
         if (active) {
@@ -445,6 +448,9 @@ __device__ __forceinline__ void search_task(const SearchArgs& A, const Hot64& H,
     if (active) {
         A.target[idx] = result;
     }
+    if (A.redo_only) {
+        return;  // counted by the form that left them
+    }
     // touched-node counter (reference-equivalent acceptance tests)
     unsigned long long t = touched;
     for (int o = 16; o > 0; o >>= 1) {
@@ -495,19 +501,16 @@ __global__ void __launch_bounds__(1024, 1) k_search_hot(SearchArgs A, uint32_t h
 }
 
 // ------------------------------------------------- one search per warp
-// (bh_wide.cuh): the FP64 evaluation, search and kernel.
-// Both signal types' search lists in one launch: the tasks of S[0] (the
-// excitatory list) first, then those of S[1]; a type without searches has no
-// tasks.  Every search waits on memory round after round, so the lists of the
-// two types share the device instead of running one launch after the other.
+// (bh_wide.cuh): the FP64 evaluation, search and kernel, over the searches
+// that the bins form (below) left at kRedo; both signal types in one launch.
 struct WideArgs {
     SearchArgs S[2];
-    uint32_t num_tasks[2];
+    const uint32_t* redo[2];  // list entries left at kRedo
     WideSlot all;        // scratch of every warp slot, `cap` entries each
     uint32_t cap;
     uint32_t slots;
     uint32_t* tasks;     // task counter over both lists
-    uint32_t* overflow;  // per type: searches left to the packet kernel
+    uint32_t* counts;    // per type: entries of redo, then those left to the packet kernel
     unsigned long long* touched;
 };
 
@@ -593,19 +596,167 @@ __device__ int32_t wide_search(const SearchArgs& S, uint32_t cap, const WideSlot
     return -1;
 }
 
-// Persistent warps, one search per task: the task counter hands out list
-// entries (32 per warp task of the packet kernels' segment layout).
+// Persistent warps, one search per task.
 template <int WPB>
 __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide(WideArgs A) {
     __shared__ uint32_t s_round_all[WPB][kWideRounds + 1];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const uint32_t slot = blockIdx.x * WPB + (uint32_t)wib;
-    if (slot >= A.slots) {
+    const uint32_t total0 = A.counts[0];
+    const uint32_t total_tasks = total0 + A.counts[1];
+    if (slot >= A.slots || total_tasks == 0u) {
         return;  // whole warp
     }
     uint32_t* s_round = s_round_all[wib];
     const WideSlot P = wide_slot(A.all, (uint64_t)slot * A.cap);
+    uint32_t touched = 0;
+    for (;;) {
+        uint32_t task = 0;
+        if (lane == 0) {
+            task = atomicAdd(A.tasks, 1u);
+        }
+        task = __shfl_sync(0xFFFFFFFFu, task, 0);
+        if (task >= total_tasks) {
+            break;
+        }
+        const int t = task < total0 ? 0 : 1;
+        const SearchArgs& S = A.S[t];
+        const uint64_t idx = A.redo[t][task - (t ? total0 : 0u)];
+        const uint32_t seg = wide_entry_segment(idx, S.seg_begin, S.num_segs);
+        const NetInfo& N = S.nets[S.seg_net[seg]];
+        const WarpNet W{ N.theta, N.scale, N.seed, S.seg_net[seg], N.first };
+        uint32_t again = 0;  // the bins form has counted this search's acceptance tests
+        const int32_t result = wide_search(S, A.cap, P, W, S.list_src[idx], S.list_j[idx], s_round, again);
+        if (lane == 0) {
+            S.target[idx] = result;
+            if (result == kRedo) {
+                atomicAdd(A.counts + 2 + t, 1u);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// ------------------------------------------------- one search per warp, by bins
+// (bh_bins.cuh): the FP64 evaluation and kernel.  Both signal types' search
+// lists in one launch: the tasks of S[0] (the excitatory list) first, then
+// those of S[1]; a type without searches has no tasks.
+struct BinsArgs {
+    SearchArgs S[2];
+    uint32_t num_tasks[2];
+    const int32_t* parent;
+    uint32_t* redo[2];
+    uint32_t levels;
+    uint32_t* tasks;   // task counter over both lists
+    uint32_t* counts;  // per type: entries of redo
+    unsigned long long* touched;
+};
+
+// Whether an inner node at (dx, dy, dz) from the source is expanded, accepted
+// or discarded, by evaluate's own operations (for the rare nodes whose test
+// is too close for the squared form).
+__device__ __noinline__ int exact_status(double dx, double dy, double dz, double md, double theta, bool leaf) {
+    const double d = rl_hypot3(dx, dy, dz);
+    if (d == 0.0) {
+        return ST_DISCARD;
+    }
+    return leaf || md < theta * d ? ST_ACCEPT : ST_EXPAND;
+}
+
+// FP64 evaluation of a node for the bins form.  SQUARED (the Gaussian kernel
+// around 0): the weight exp(-d^2 / sigma^2) and the test md^2 < theta^2 d^2
+// need no square root, so a node costs 17 FP64 operations instead of the 55 of
+// evaluate's hypot and exp.  The status is evaluate's: a test within 2e-6 of
+// equality, which the FP32 operands (each within 2^-24, the squares and
+// products within 6 x 2^-24 together) cannot decide, is made by exact_status.
+// The weight differs from evaluate's by less than 1e-11 of itself wherever it
+// counts (kBinsMargin64).  Otherwise evaluate itself.
+template <bool SQUARED>
+struct Bins64 {
+    const SearchArgs& S;
+    const WarpNet& W;
+    const double4* __restrict__ rec;
+    const uint4* __restrict__ meta;
+    const double* tab;  // 2^(j/64) in shared memory
+    double sx, sy, sz;
+    double to_k;  // -64 / (ln 2 sigma^2)
+    float theta2;
+    uint32_t source, num_nodes;
+
+    __device__ __forceinline__ BinsEval operator()(uint32_t nd) const {
+        BinsEval e{ ST_DISCARD, 0.0, 0u, 0u, false };
+        if (nd >= num_nodes) {
+            return e;
+        }
+        const uint4 mm = __ldg(&meta[nd]);
+        const double4 rr = ldg4(&rec[nd]);
+        const bool leaf = topo_leaf(mm.y);
+        if constexpr (!SQUARED) {
+            const Eval ev = evaluate(rr, make_uint2(mm.x, mm.y), __ldg(&S.maxdim[nd]), sx, sy, sz, source, W.theta, S.mu, W.scale, false, S.kernel);
+            e.status = ev.status;
+            e.w = ev.w;
+            e.cand = ev.status == ST_ACCEPT && !(leaf && mm.x == source);
+        } else {
+            const uint32_t cnt = rcount(rr);
+            if (cnt == 0u || (leaf && mm.x == source)) {
+                return e;  // the source itself weighs 0: as good as discarded
+            }
+            const double dx = rr.x - sx, dy = rr.y - sy, dz = rr.z - sz;
+            const double d2 = __fma_rn(dx, dx, __fma_rn(dy, dy, dz * dz));
+            const float md = __uint_as_float(mm.w);
+            const float m2 = md * md, t2 = theta2 * (float)d2;
+            int status = leaf || m2 < t2 ? ST_ACCEPT : ST_EXPAND;
+            if ((!leaf && fabsf(m2 - t2) <= 2e-6f * m2) || d2 < 1e-200) {
+                status = exact_status(dx, dy, dz, __ldg(&S.maxdim[nd]), W.theta, leaf);
+            }
+            e.status = status;
+            if (status == ST_ACCEPT) {
+                // 2^(k/64) e^s with k the nearest integer (1.5 x 2^52 rounds it), |s| < 0.0055:
+                // Tang's reduction as in rl_exp, to 4e-14 of the value
+                const double km = __fma_rn(d2, to_k, 6755399441055744.0);
+                const double kd = km - 6755399441055744.0;
+                const double x = d2 * W.scale;
+                const double s = __fma_rn(kd, -0.010830424696249145, x);  // ln 2 / 64
+                double q = __fma_rn(s, 1.0 / 24.0, 1.0 / 6.0);
+                q = __fma_rn(q, s, 0.5);
+                q = __fma_rn(q, s, 1.0);
+                const int k = __double2loint(km);
+                const double t = tab[k & 63];
+                const double t2m = __hiloint2double(__double2hiint(t) + ((k >> 6) << 20), __double2loint(t));
+                const double w = __fma_rn(t2m * s, q, t2m);
+                e.w = x < -700.0 ? 0.0 : w * (double)cnt;
+                e.cand = true;
+            }
+        }
+        if (e.status == ST_EXPAND) {
+            e.first = mm.x;
+            e.nch = (uint32_t)__popc(topo_mask(mm.y));
+        }
+        return e;
+    }
+};
+
+// Bound on the difference between the bins form's running sums (and r) and
+// the reference's, relative to the total T of v visited nodes: additions of
+// positive terms in any order are within v 2^-53 of the sum, on both sides
+// and for r as well; the squared form's weights are within |x| 8 x 2^-53 of
+// evaluate's for an exponent x (|x| <= 700) plus 4e-14.  Totals below kBinsTiny
+// (dropped weights, exponents below -700) are left to the ordered form.
+constexpr double kBinsMargin64 = 2e-11;
+constexpr double kBinsTiny64 = 1e-250;
+
+template <int WPB, bool SQUARED>
+__global__ void __launch_bounds__(WPB * 32, SQUARED ? 20 / WPB : 16 / WPB) k_search_bins(BinsArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_bins[];
+    double* tab = reinterpret_cast<double*>(smem_bins);
+    for (uint32_t i = threadIdx.x; i < 64u; i += WPB * 32) {
+        tab[i] = rl_exp_table_dev[i].x;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    const BinsMem M = bins_mem(smem_bins + 64 * sizeof(double) + (size_t)wib * bins_warp_bytes(A.levels), A.levels);
     const uint32_t total0 = A.num_tasks[0];
     const uint32_t total_tasks = total0 + A.num_tasks[1];
     uint32_t touched = 0;
@@ -629,12 +780,18 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide(WideArgs A) {
         const WarpNet W{ N.theta, N.scale, N.seed, S.seg_net[lo], N.first };
         int32_t result = -1;
         if (!N.root_leaf) {
-            result = wide_search(S, A.cap, P, W, S.list_src[idx], S.list_j[idx], s_round, touched);
+            const uint32_t source = S.list_src[idx];
+            const uint32_t j = S.list_j[idx];
+            const Bins64<SQUARED> ev{ S, W, S.rec, S.meta, tab, S.px[source], S.py[source], S.pz[source], W.scale * 92.332482616893656768, (float)(W.theta * W.theta),
+                                      source, S.num_nodes };
+            result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny64, touched, ev,
+                                 [&](double total, uint32_t depth) { return pick_threshold(total, W.seed, S.step, source - W.first, j, depth); },
+                                 [&](double total, uint32_t visited) { return total * (kBinsMargin64 + (double)visited * 4.5e-16); });
         }
         if (lane == 0) {
             S.target[idx] = result;
             if (result == kRedo) {
-                atomicAdd(A.overflow + t, 1u);
+                A.redo[t][atomicAdd(A.counts + t, 1u)] = (uint32_t)idx;
             }
         }
         __syncwarp();
@@ -784,55 +941,125 @@ WideSlot wide_scratch(Ctx& c, uint32_t slots, uint32_t cap) {
     return WideSlot{ S.w_node.p, S.w_info.p, S.w_child.p, S.w_cnt.p, S.w_pos.p, S.w_ord_node.p, S.w_w.p, S.w_ord_w.p };
 }
 
-// Whether the tuner times a candidate shape on this context's search list:
-// the one-search-per-warp form pays off on large networks with sparse lists
-// only (on a dense list its scratch would hold a warp slot per resident warp
-// for nothing: packets of Morton neighbours are several times faster there).
-bool search_variant_applies(const Ctx& c, const SearchVariant& v) {
-    return v.packet != 0 || (c.n >= kWideMinNeurons && search_density_class(c.n, c.search.num_searches) != 0);
-}
-
 namespace {
 
-// The one-search-per-warp kernel on both signal types' lists (warps[t]
-// packet-layout warps of type t, 0 for a type without searches); a type with
-// searches that did not fit their warp's scratch is redone by the packet
-// kernel (which writes every target of its list again).
-void launch_wide(Ctx& c, const SearchArgs (&a)[2], const uint32_t (&warps)[2]) {
+// Whether the bins form can take the squared FP64 evaluation (Bins64): the
+// Gaussian kernel around 0, and boxes whose squared lengths and cells (down to
+// the deepest level) are normal FP32 numbers.
+bool bins_squared(const Ctx& c) {
+    if (c.kernel.type != RL_KERNEL_GAUSSIAN || c.cfg.mu != 0.0) {
+        return false;
+    }
+    for (const NetInfo& N : c.nets) {
+        if (!(N.theta >= 1e-4 && N.sigma >= 1e-9 && N.sigma <= 1e15)) {
+            return false;
+        }
+        for (int k = 0; k < 3; ++k) {
+            const double edge = N.box_max[k] - N.box_min[k];
+            if (!(edge >= 1e-2 && edge <= 1e15 && std::fabs(N.box_min[k]) <= 1e15)) {
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
+template <bool SQUARED>
+void launch_bins_kernel(Ctx& c, const BinsArgs& A) {
     constexpr int WPB = 4;
+    auto kern = &k_search_bins<WPB, SQUARED>;
+    const size_t smem = 64 * sizeof(double) + WPB * bins_warp_bytes(A.levels);
+    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kern, WPB * 32, smem));
+    const uint32_t tasks = A.num_tasks[0] + A.num_tasks[1];
+    const uint32_t blocks = std::min<uint32_t>((tasks + WPB - 1) / WPB, (uint32_t)std::max(per_sm, 1) * (uint32_t)c.num_sms);
+    kern<<<blocks, WPB * 32, smem, c.stream>>>(A);
+    RL_LAUNCH_CHECK();
+}
+
+// One search per warp on both signal types' lists (warps[t] packet-layout
+// warps of type t, 0 for a type without searches): the bins form, then the
+// searches it left open in the reference's order — one warp each, or by the
+// packet kernel where they are many (every total underflowed) or did not fit
+// their warp's scratch.
+void launch_wide(Ctx& c, const SearchArgs (&a)[2], const uint32_t (&warps)[2]) {
     Search& S = c.search;
     cudaStream_t st = c.stream;
-    const uint32_t tasks = (warps[0] + warps[1]) * 32u;
-    const uint32_t cap = wide_cap(c);
-    const uint32_t slots = std::min<uint32_t>(tasks, (uint32_t)c.num_sms * kWideWarpsPerSM);
-    S.w_overflow.ensure(2);
+    S.w_counts.ensure(4);
+    S.w_redo.ensure(S.num_searches);
     RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), st));
-    RL_CUDA_TRY(cudaMemsetAsync(S.w_overflow.p, 0, 2 * sizeof(uint32_t), st));
-    WideArgs A;
-    for (int t = 0; t < 2; ++t) {
-        A.S[t] = a[t];
-        A.num_tasks[t] = warps[t] * 32u;
+    RL_CUDA_TRY(cudaMemsetAsync(S.w_counts.p, 0, 4 * sizeof(uint32_t), st));
+    uint32_t* redo[2] = { S.w_redo.p, S.w_redo.p + S.num_exc };
+    {
+        BinsArgs A;
+        for (int t = 0; t < 2; ++t) {
+            A.S[t] = a[t];
+            A.num_tasks[t] = warps[t] * 32u;
+            A.redo[t] = redo[t];
+        }
+        A.parent = c.tree.parent.p;
+        A.levels = std::max(c.tree.max_level, 1u);
+        A.tasks = S.tasks.p;
+        A.counts = S.w_counts.p;
+        A.touched = reinterpret_cast<unsigned long long*>(c.counters.p);
+        if (bins_squared(c)) {
+            launch_bins_kernel<true>(c, A);
+        } else {
+            launch_bins_kernel<false>(c, A);
+        }
     }
-    A.all = wide_scratch(c, slots, cap);
-    A.cap = cap;
-    A.slots = slots;
-    A.tasks = S.tasks.p;
-    A.overflow = S.w_overflow.p;
-    A.touched = reinterpret_cast<unsigned long long*>(c.counters.p);
-    k_search_wide<WPB><<<(slots + WPB - 1) / WPB, WPB * 32, 0, st>>>(A);
-    RL_LAUNCH_CHECK();
-    uint32_t over[2] = { 0, 0 };
-    RL_CUDA_TRY(cudaMemcpyAsync(over, S.w_overflow.p, sizeof(over), cudaMemcpyDeviceToHost, st));
+    uint32_t left[4] = { 0, 0, 0, 0 };
+    RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     RL_CUDA_TRY(cudaStreamSynchronize(st));
+    const uint64_t open = (uint64_t)left[0] + left[1];
+    if (open == 0) {
+        return;
+    }
+    if (!wide_redo_by_packets(c, open)) {
+        constexpr int WPB = 4;
+        const uint32_t cap = wide_cap(c);
+        const uint32_t slots = (uint32_t)std::min<uint64_t>(open, (uint64_t)c.num_sms * kWideWarpsPerSM);
+        RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), st));
+        WideArgs A;
+        for (int t = 0; t < 2; ++t) {
+            A.S[t] = a[t];
+            A.redo[t] = redo[t];
+        }
+        A.all = wide_scratch(c, slots, cap);
+        A.cap = cap;
+        A.slots = slots;
+        A.tasks = S.tasks.p;
+        A.counts = S.w_counts.p;
+        A.touched = reinterpret_cast<unsigned long long*>(c.counters.p);
+        k_search_wide<WPB><<<(slots + WPB - 1) / WPB, WPB * 32, 0, st>>>(A);
+        RL_LAUNCH_CHECK();
+        RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p + 2, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        RL_CUDA_TRY(cudaStreamSynchronize(st));
+    }
     for (int t = 0; t < 2; ++t) {
-        if (over[t]) {
-            k_search<2, 32, 1><<<(warps[t] + 1) / 2, 64, 0, st>>>(a[t]);
+        if (left[t]) {
+            SearchArgs p = a[t];
+            p.redo_only = 1;
+            k_search<2, 32, 1><<<(warps[t] + 1) / 2, 64, 0, st>>>(p);
             RL_LAUNCH_CHECK();
         }
     }
 }
 
 }  // namespace
+
+// Whether the tuner times a candidate shape on this context's search list.
+bool search_variant_applies(const Ctx&, const SearchVariant&) {
+    return true;
+}
+
+// Searches that the bins form left open go one per warp, unless a large share
+// of a dense list is open (totals that underflow): then packets of Morton
+// neighbours are faster.
+bool wide_redo_by_packets(const Ctx& c, uint64_t open) {
+    return open > 4096 && 8 * open > c.search.num_searches && search_density_class(c.n, c.search.num_searches) == 0;
+}
 
 // Times every search variant that fits the octree on the current search list
 // and keeps the fastest.  Each variant runs twice (the second run is timed);
@@ -1034,6 +1261,7 @@ void run_search(Ctx& c, uint32_t step) {
             A.err = c.err.p;
             A.touched = reinterpret_cast<unsigned long long*>(c.counters.p);
             A.kernel = c.kernel;
+            A.redo_only = 0;
         }
         auto launch_all = [&](const SearchVariant& v) {
             if (v.packet == 0) {

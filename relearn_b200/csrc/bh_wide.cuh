@@ -24,7 +24,8 @@
 //     is the first partial sum that reaches r.
 // Deeper descents run the same way from the picked node.  A warp's scratch
 // holds `cap` walk entries; a search that does not fit is left to the packet
-// kernel (target kRedo).
+// kernel (target kRedo).  This is the form for searches whose pick depends on
+// the order of the additions (bh_bins.cuh sends them here).
 #pragma once
 
 #include "rl_context.cuh"
@@ -277,6 +278,20 @@ __device__ __forceinline__ int64_t wide_pick(const double* ord_w, const uint32_t
         }
     }
     return -1;
+}
+
+// The segment of list entry idx.
+__device__ __forceinline__ uint32_t wide_entry_segment(uint64_t idx, const uint64_t* seg_begin, uint32_t num_segs) {
+    uint32_t lo = 0, hi = num_segs;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (seg_begin[mid] <= idx) {
+            lo = mid;
+        } else {
+            hi = mid;
+        }
+    }
+    return lo;
 }
 
 // The list entry of wide task `task` (32 tasks per warp task of the packet

@@ -22,8 +22,8 @@
 // Errors against the FP64 form are measured, not assumed (bench.py
 // --precision-report): selection probabilities, calcium drift, distances of
 // formed synapses.
+#include "bh_bins.cuh"
 #include "bh_eval.cuh"
-#include "bh_wide.cuh"
 #include "rl_context.cuh"
 #include "rl_math.cuh"
 
@@ -746,6 +746,7 @@ struct Search32 {
     uint32_t step;
     uint32_t* err;
     Kernel32 kernel;
+    int redo_only;  // packet kernel: only the list entries left at kRedo
 };
 
 // Parameters of the network a warp searches in.
@@ -1039,7 +1040,7 @@ __device__ __forceinline__ void search_task32(const Search32& A, const Hot32& H,
     const NetInfo& N = A.nets[A.seg_net[lo]];
     const Net32 W{ N.theta32, N.inv_sigma2_32, N.seed, A.seg_net[lo], N.first, N.frame.quantum };
     const uint64_t idx = A.seg_begin[lo] + (uint64_t)(warp_global - A.seg_warp[lo]) * 32 + lane;
-    const bool active = idx < A.seg_end[lo];
+    const bool active = idx < A.seg_end[lo] && (!A.redo_only || A.target[idx] == kRedo);
     if (N.root_leaf) {
         if (active) {
             A.target[idx] = -1;
@@ -1179,17 +1180,17 @@ __global__ void __launch_bounds__(1024, 1) k_search_f32_hot(Search32 A, uint32_t
     }
 }
 
-// One search per warp (bh_wide.cuh) in the FP32 form: the same visiting
-// order and the same Kahan sums as the packet kernels, so the same targets.
-// Both signal types' lists in one launch (the FP64 form's WideArgs).
+// One search per warp in the reference's order (bh_wide.cuh) in the FP32
+// form: the same visiting order and the same Kahan sums as the packet kernels,
+// so the same targets; over the searches the bins form left at kRedo.
 struct WideArgs32 {
     Search32 S[2];
-    uint32_t num_tasks[2];
+    const uint32_t* redo[2];  // list entries left at kRedo
     WideSlot all;
     uint32_t cap;
     uint32_t slots;
     uint32_t* tasks;
-    uint32_t* overflow;  // per type
+    uint32_t* counts;  // per type: entries of redo, then those left to the packet kernel
 };
 
 __device__ int32_t wide_search32(const Search32& S, uint32_t cap, const WideSlot& P, const Net32& W, const QPos& sp, uint32_t source, uint32_t j,
@@ -1263,14 +1264,74 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide32(WideArgs32 A) {
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const uint32_t slot = blockIdx.x * WPB + (uint32_t)wib;
-    if (slot >= A.slots) {
+    const uint32_t total0 = A.counts[0];
+    const uint32_t total_tasks = total0 + A.counts[1];
+    if (slot >= A.slots || total_tasks == 0u) {
         return;  // whole warp
     }
     const uint64_t off = (uint64_t)slot * A.cap;
     const WideSlot P{ A.all.node + off, A.all.info + off, A.all.child + off, A.all.cnt + off, A.all.pos + off, A.all.ord_node + off, A.all.w + off,
                       A.all.ord_w + off };
+    for (;;) {
+        uint32_t task = 0;
+        if (lane == 0) {
+            task = atomicAdd(A.tasks, 1u);
+        }
+        task = __shfl_sync(0xFFFFFFFFu, task, 0);
+        if (task >= total_tasks) {
+            break;
+        }
+        const int t = task < total0 ? 0 : 1;
+        const Search32& S = A.S[t];
+        const uint64_t idx = A.redo[t][task - (t ? total0 : 0u)];
+        const uint32_t seg = wide_entry_segment(idx, S.seg_begin, S.num_segs);
+        const NetInfo& N = S.nets[S.seg_net[seg]];
+        const Net32 W{ N.theta32, N.inv_sigma2_32, N.seed, S.seg_net[seg], N.first, N.frame.quantum };
+        const uint32_t source = S.list_src[idx];
+        const QFrame& F = N.frame;
+        const QPos sp{ quantize(S.px[source], F.origin[0], F.inv_quantum), quantize(S.py[source], F.origin[1], F.inv_quantum),
+                       quantize(S.pz[source], F.origin[2], F.inv_quantum) };
+        const int32_t result = wide_search32(S, A.cap, P, W, sp, source, S.list_j[idx], s_round_all[wib]);
+        if (lane == 0) {
+            S.target[idx] = result;
+            if (result == kRedo) {
+                atomicAdd(A.counts + 2 + t, 1u);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// One search per warp by sums over bins (bh_bins.cuh) in the FP32 form: every
+// node's status and weight are eval32's bits, the bins are summed in FP64.
+// Both signal types' lists in one launch, as in the FP64 form.
+struct BinsArgs32 {
+    Search32 S[2];
+    uint32_t num_tasks[2];
+    const int32_t* parent;
+    uint32_t* redo[2];
+    uint32_t levels;
+    uint32_t* tasks;
+    uint32_t* counts;  // per type: entries of redo
+};
+
+// The Kahan sums of n FP32 weights lie within (2 + n 2^-24) 2^-24 of the exact
+// ones, r within 3 x 2^-24 of the exact total's share (its total and one
+// rounding), and the bins' FP64 sums within n 2^-53: 5.1 x 2^-24 of the total
+// together for any n that fits an octree.  Totals below kBinsTiny32 (weights
+// in the subnormal range) are left to the ordered form.
+constexpr double kBinsMargin32 = 3.3e-7;
+constexpr double kBinsTiny32 = 1e-30;
+
+template <int WPB>
+__global__ void __launch_bounds__(WPB * 32, 32 / WPB) k_search_bins32(BinsArgs32 A) {
+    extern __shared__ __align__(16) unsigned char smem_bins[];
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    const BinsMem M = bins_mem(smem_bins + (size_t)wib * bins_warp_bytes(A.levels), A.levels);
     const uint32_t total0 = A.num_tasks[0];
     const uint32_t total_tasks = total0 + A.num_tasks[1];
+    uint32_t touched = 0;
     for (;;) {
         uint32_t task = 0;
         if (lane == 0) {
@@ -1292,15 +1353,39 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide32(WideArgs32 A) {
         int32_t result = -1;
         if (!N.root_leaf) {
             const uint32_t source = S.list_src[idx];
+            const uint32_t j = S.list_j[idx];
             const QFrame& F = N.frame;
             const QPos sp{ quantize(S.px[source], F.origin[0], F.inv_quantum), quantize(S.py[source], F.origin[1], F.inv_quantum),
                            quantize(S.pz[source], F.origin[2], F.inv_quantum) };
-            result = wide_search32(S, A.cap, P, W, sp, source, S.list_j[idx], s_round_all[wib]);
+            auto ev = [&](uint32_t nd) {
+                BinsEval r{ S_DISCARD, 0.0, 0u, 0u, false };
+                if (nd >= S.num_nodes) {
+                    return r;
+                }
+                const uint4 mm = __ldg(&S.meta[nd]);
+                const E32 e = eval32(__ldg(&S.rec[nd]), mtopo(mm), mmaxdim(mm), sp, source, S, W, false);
+                r.status = e.status;
+                if (e.status == S_ACCEPT) {
+                    r.w = (double)e.w;
+                    r.cand = !(topo_leaf(mm.y) && mm.x == source);
+                } else if (e.status == S_EXPAND) {
+                    r.first = mm.x;
+                    r.nch = (uint32_t)__popc(topo_mask(mm.y));
+                }
+                return r;
+            };
+            result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny32, touched, ev,
+                                 [&](double total, uint32_t depth) {
+                                     const u32x4 w = draw(W.seed, S.step, source - W.first, j, STREAM_BH_PICK, depth);  // as threshold32
+                                     const double r = (double)(w.x >> 8) * 5.9604644775390625e-8 * total;
+                                     return r > 0.0 ? r : 1.0e-38;
+                                 },
+                                 [&](double total, uint32_t) { return total * kBinsMargin32; });
         }
         if (lane == 0) {
             S.target[idx] = result;
             if (result == kRedo) {
-                atomicAdd(A.overflow + t, 1u);
+                A.redo[t][atomicAdd(A.counts + t, 1u)] = (uint32_t)idx;
             }
         }
         __syncwarp();
@@ -1673,6 +1758,7 @@ Search32 search32_args(Ctx& c, int type, const uint32_t* seg_warp, const uint64_
     A.step = step;
     A.err = c.err.p;
     A.kernel = Kernel32{ c.kernel.type, c.kernel.cutoff_inf, (float)c.kernel.k_minus_1, (float)c.kernel.a, (float)c.kernel.b, (float)c.kernel.cutoff };
+    A.redo_only = 0;
     return A;
 }
 
@@ -1701,36 +1787,69 @@ void launch_search_f32(Ctx& c, int type, const uint32_t* seg_warp, const uint64_
 
 // One search per warp over both signal types' lists (warps[t] packet-layout
 // warps of type t, 0 for a type without searches, num_segs[t] segments in
-// c.search.seg_*[t]); a type with searches that did not fit their warp's
-// scratch is redone by the packet kernel.
+// c.search.seg_*[t]): the bins form, then the searches it left open, as in the
+// FP64 form.
 void launch_search_wide_f32(Ctx& c, const uint32_t (&warps)[2], uint32_t segs0, uint32_t segs1, uint32_t step) {
     constexpr int WPB = 4;
     Search& S = c.search;
     const uint32_t segs[2] = { segs0, segs1 };
-    WideArgs32 W;
-    for (int t = 0; t < 2; ++t) {
-        W.S[t] = warps[t] ? search32_args(c, t, S.seg_warp[t].p, S.seg_begin[t].p, S.seg_end[t].p, S.seg_net[t].p, segs[t], step, S.tasks.p + t)
-                          : Search32{};
-        W.num_tasks[t] = warps[t] * 32u;
-    }
-    const uint32_t cap = wide_cap(c);
-    const uint32_t slots = std::min<uint32_t>((warps[0] + warps[1]) * 32u, (uint32_t)c.num_sms * kWideWarpsPerSM);
-    S.w_overflow.ensure(2);
+    S.w_counts.ensure(4);
+    S.w_redo.ensure(S.num_searches);
     RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), c.stream));
-    RL_CUDA_TRY(cudaMemsetAsync(S.w_overflow.p, 0, 2 * sizeof(uint32_t), c.stream));
-    W.all = wide_scratch(c, slots, cap);
-    W.cap = cap;
-    W.slots = slots;
-    W.tasks = S.tasks.p;
-    W.overflow = S.w_overflow.p;
-    k_search_wide32<WPB><<<(slots + WPB - 1) / WPB, WPB * 32, 0, c.stream>>>(W);
-    RL_LAUNCH_CHECK();
-    uint32_t over[2] = { 0, 0 };
-    RL_CUDA_TRY(cudaMemcpyAsync(over, S.w_overflow.p, sizeof(over), cudaMemcpyDeviceToHost, c.stream));
-    RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    RL_CUDA_TRY(cudaMemsetAsync(S.w_counts.p, 0, 4 * sizeof(uint32_t), c.stream));
+    BinsArgs32 B;
     for (int t = 0; t < 2; ++t) {
-        if (over[t]) {
-            k_search_f32<2, 32, 1><<<(warps[t] + 1) / 2, 64, 0, c.stream>>>(W.S[t]);
+        B.S[t] = warps[t] ? search32_args(c, t, S.seg_warp[t].p, S.seg_begin[t].p, S.seg_end[t].p, S.seg_net[t].p, segs[t], step, S.tasks.p + t)
+                          : Search32{};
+        B.num_tasks[t] = warps[t] * 32u;
+        B.redo[t] = S.w_redo.p + (t ? S.num_exc : 0);
+    }
+    B.parent = c.tree.parent.p;
+    B.levels = std::max(c.tree.max_level, 1u);
+    B.tasks = S.tasks.p;
+    B.counts = S.w_counts.p;
+    {
+        auto kern = &k_search_bins32<WPB>;
+        const size_t smem = WPB * bins_warp_bytes(B.levels);
+        RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int per_sm = 0;
+        RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kern, WPB * 32, smem));
+        const uint32_t tasks = B.num_tasks[0] + B.num_tasks[1];
+        const uint32_t blocks = std::min<uint32_t>((tasks + WPB - 1) / WPB, (uint32_t)std::max(per_sm, 1) * (uint32_t)c.num_sms);
+        kern<<<blocks, WPB * 32, smem, c.stream>>>(B);
+        RL_LAUNCH_CHECK();
+    }
+    uint32_t left[4] = { 0, 0, 0, 0 };
+    RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+    RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    const uint64_t open = (uint64_t)left[0] + left[1];
+    if (open == 0) {
+        return;
+    }
+    if (!wide_redo_by_packets(c, open)) {
+        const uint32_t cap = wide_cap(c);
+        const uint32_t slots = (uint32_t)std::min<uint64_t>(open, (uint64_t)c.num_sms * kWideWarpsPerSM);
+        RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), c.stream));
+        WideArgs32 W;
+        for (int t = 0; t < 2; ++t) {
+            W.S[t] = B.S[t];
+            W.redo[t] = B.redo[t];
+        }
+        W.all = wide_scratch(c, slots, cap);
+        W.cap = cap;
+        W.slots = slots;
+        W.tasks = S.tasks.p;
+        W.counts = S.w_counts.p;
+        k_search_wide32<WPB><<<(slots + WPB - 1) / WPB, WPB * 32, 0, c.stream>>>(W);
+        RL_LAUNCH_CHECK();
+        RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p + 2, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+        RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    }
+    for (int t = 0; t < 2; ++t) {
+        if (left[t]) {
+            Search32 p = B.S[t];
+            p.redo_only = 1;
+            k_search_f32<2, 32, 1><<<(warps[t] + 1) / 2, 64, 0, c.stream>>>(p);
             RL_LAUNCH_CHECK();
         }
     }

@@ -128,8 +128,10 @@ struct Search {
     DBuf<uint32_t> seg_warp[2], seg_net[2];
     DBuf<uint64_t> seg_begin[2], seg_end[2];
     // one-search-per-warp form: walk entries of every warp slot
-    DBuf<uint32_t> w_node, w_info, w_child, w_cnt, w_pos, w_ord_node, w_overflow;
+    DBuf<uint32_t> w_node, w_info, w_child, w_cnt, w_pos, w_ord_node;
     DBuf<double> w_w, w_ord_w;
+    // searches the bins form left to the ordered form, per signal type, and their counts
+    DBuf<uint32_t> w_redo, w_counts;
     uint64_t num_searches = 0;
     uint64_t num_exc = 0;
     uint64_t num_requests = 0;
@@ -310,13 +312,13 @@ struct Tuning {
 
 const std::vector<SearchVariant>& search_variants();
 bool search_variant_applies(const Ctx& c, const SearchVariant& v);
+bool wide_redo_by_packets(const Ctx& c, uint64_t open);
 struct WideSlot;
 uint32_t wide_cap(const Ctx& c);
 WideSlot wide_scratch(Ctx& c, uint32_t slots, uint32_t cap);
-// one-search-per-warp form: walk entries per warp, warps per SM, smallest network
+// one search per warp in the reference's order: walk entries per warp, warps per SM
 constexpr uint32_t kWideCap = 6144;
 constexpr uint32_t kWideWarpsPerSM = 16;
-constexpr uint32_t kWideMinNeurons = 65536;
 uint32_t hot_nodes(const Ctx& c, const SearchVariant& v, size_t node_bytes);
 const std::vector<ActVariant>& act_variants();
 
