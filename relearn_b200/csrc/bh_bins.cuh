@@ -21,9 +21,6 @@
 // bin's subtree (a few dozen nodes) is walked again, with a bin per child,
 // down to the candidate.
 //
-// Bound: instruction issue.  About 200 passes of 85 instructions per search
-// at 1M neurons; node records come from L1 (neighbouring warps search for
-// Morton-adjacent sources).
 #pragma once
 
 #include "bh_wide.cuh"
@@ -32,11 +29,17 @@ namespace rl {
 
 constexpr uint32_t kBinCopies = 4;  // one per group of 8 lanes, so that groups never add to the same word
 
+// What ev(node, act) returns.  Every lane evaluates (one without a node, act
+// false, evaluates node 0), and the results are selected: with branches the
+// lanes of a pass run the accepting, the expanding and the idle path one after
+// the other (200,000 searches of 200,000 neurons, FP64 / FP32: 4.96e9 / 4.35e9
+// warp instructions and 7.4 / 6.3 ms with branches, 4.43e9 / 3.51e9 and 5.6 /
+// 4.2 ms selected).
 struct BinsEval {
-    int status;      // 0 discard, 1 expand, 2 accept (ST_* / S_*)
     double w;        // weight of an accepted node, else 0
-    uint32_t first;  // an expanded node's first child
+    uint32_t first;  // first child (of a node that expands)
     uint32_t nch;    // and its children
+    bool expand;
     bool cand;       // accepted and not the source itself
 };
 
@@ -51,10 +54,12 @@ struct BinsMem {
     uint32_t cap;           // stack entries
 };
 
-// A batch of four entries pushes at most 32 and pops four, one level deeper
-// each time (28 per level), on top of the chain's at most 7 per level.
+// The chain leaves at most 7 entries per level; on top of them a batch of four
+// pops four entries and pushes as many on average (32 at most, one level
+// deeper).  The room is kept small, since it comes out of the L1 cache that
+// holds the octree; a search that needs more goes to the ordered form.
 __host__ __device__ __forceinline__ uint32_t bins_stack_cap(uint32_t levels) {
-    return 35u * levels + 34u;
+    return 12u * levels + 96u;
 }
 __host__ __device__ __forceinline__ size_t bins_warp_bytes(uint32_t levels) {
     const size_t b = (size_t)kBinCopies * 8u * levels * sizeof(double) + (size_t)bins_stack_cap(levels) * sizeof(uint2) + (3u * (size_t)levels + 1u) * sizeof(uint32_t);
@@ -74,44 +79,38 @@ __device__ __forceinline__ BinsMem bins_mem(unsigned char* p, uint32_t levels) {
 }
 
 // Empties the stack of `top` entries into the bins; false if it would
-// overflow or a node lies outside the octree (the ordered form reports that).
+// overflow or the walk visits more nodes than there are (the ordered form
+// reports that).
 template <class Ev>
 __device__ __forceinline__ bool bins_drain(const BinsMem& M, uint32_t top, uint32_t num_nodes, uint32_t& touched, bool& any, Ev&& ev) {
     const uint32_t lane = threadIdx.x & 31u, g = lane >> 3, sub = lane & 7u;
     const uint32_t below = (1u << lane) - 1u;
     double* mine = M.bin + g * M.nb;
-    uint32_t guard = 0;
-    while (top > 0) {
-        const uint32_t take = top < 4u ? top : 4u;
-        BinsEval e{ 0, 0.0, 0u, 0u, false };
-        uint32_t bin = 0;
-        const bool have = g < take;
-        if (have) {
-            const uint2 s = M.stack[top - 1u - g];
-            bin = s.y & 0xFFFFu;
-            if (sub < (s.y >> 16)) {
-                e = ev(s.x + sub);
-                ++touched;
-            }
-        }
-        top -= take;
+    uint32_t guard = num_nodes;
+    while (top > 0u) {
+        const uint2 s = M.stack[g < top ? top - 1u - g : 0u];
+        const bool act = g < top && sub < (s.y >> 16);
+        const BinsEval e = ev(s.x + sub, act);
+        touched += act ? 1u : 0u;
         any = any || e.cand;
         double v = e.w;
         v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
         v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
         v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
-        if (have && sub == 0u) {
+        const uint32_t bin = s.y & 0xFFFFu;
+        if (sub == 0u && g < top) {
             mine[bin] += v;
         }
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, e.status == 1);
-        const uint32_t k = (uint32_t)__popc(m);
-        if (top + k > M.cap || ++guard > num_nodes) {
+        top -= top < 4u ? top : 4u;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, e.expand);
+        const uint32_t at = top + (uint32_t)__popc(m & below);
+        top += (uint32_t)__popc(m);
+        if (top > M.cap || guard-- == 0u) {
             return false;
         }
-        if (e.status == 1) {
-            M.stack[top + (uint32_t)__popc(m & below)] = make_uint2(e.first, bin | (e.nch << 16));
+        if (e.expand) {
+            M.stack[at] = make_uint2(e.first, bin | (e.nch << 16));
         }
-        top += k;
         __syncwarp();
     }
     return true;
@@ -124,27 +123,24 @@ template <class Ev>
 __device__ __forceinline__ bool bins_children(const BinsMem& M, uint32_t first, uint32_t nch, uint32_t num_nodes, uint32_t& touched, bool& any, Ev&& ev,
                                               BinsEval& mine, double& sum) {
     const uint32_t lane = threadIdx.x & 31u, g = lane >> 3, sub = lane & 7u;
-    mine = BinsEval{ 0, 0.0, 0u, 0u, false };
-    if (lane < nch) {
-        mine = ev(first + lane);
-        ++touched;
-    }
+    mine = ev(first + lane, lane < nch);
+    touched += lane < nch ? 1u : 0u;
     any = any || mine.cand;
-    M.bin[g * M.nb + sub] = mine.w;  // lanes 0..7: the accepted children; the other copies start at 0
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine.status == 1);
-    if (mine.status == 1) {
+    sum = mine.w;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine.expand);
+    if (m == 0u) {
+        return true;
+    }
+    M.bin[g * M.nb + sub] = 0.0;
+    if (mine.expand) {
         M.stack[__popc(m & ((1u << lane) - 1u))] = make_uint2(mine.first, lane | (mine.nch << 16));
     }
     __syncwarp();
-    sum = 0.0;
-    if (m != 0u && !bins_drain(M, (uint32_t)__popc(m), num_nodes, touched, any, ev)) {
+    if (!bins_drain(M, (uint32_t)__popc(m), num_nodes, touched, any, ev)) {
         return false;
     }
-    if (lane < nch) {
-#pragma unroll
-        for (uint32_t c = 0; c < kBinCopies; ++c) {
-            sum += M.bin[c * M.nb + lane];
-        }
+    if (mine.expand) {
+        sum = ((M.bin[lane] + M.bin[M.nb + lane]) + M.bin[2u * M.nb + lane]) + M.bin[3u * M.nb + lane];
     }
     __syncwarp();
     return true;
@@ -174,8 +170,7 @@ __device__ __forceinline__ int64_t bins_pick(const BinsMem& M, uint32_t first, u
         if (hit < 0) {
             return kPickRedo;
         }
-        const int status = __shfl_sync(0xFFFFFFFFu, mine.status, hit);
-        if (status != 1) {
+        if (!__shfl_sync(0xFFFFFFFFu, mine.expand ? 1 : 0, hit)) {
             return r - pre > margin && post - r > margin ? (int64_t)(first + (uint32_t)hit) : kPickRedo;
         }
         const uint32_t f = __shfl_sync(0xFFFFFFFFu, mine.first, hit);
@@ -193,7 +188,7 @@ __device__ __forceinline__ int64_t bins_pick(const BinsMem& M, uint32_t first, u
 
 // One search by the whole warp: the target neuron, -1 when the search fails,
 // kRedo when it is left to the ordered form.
-//   ev(node)           evaluates a node
+//   ev(node, act)      evaluates a node (BinsEval)
 //   threshold(T, d)    r of descent d for the total T
 //   margin(T, visited) bound on |our running sums - the reference's| + |our r - the reference's|
 //   tiny               totals below it (weights that underflow) are left to the ordered form
@@ -229,18 +224,15 @@ __device__ int32_t bins_search(const BinsMem& M, const uint4* __restrict__ meta,
     uint32_t top = 0, levels = 0;
     for (uint32_t l0 = 0; l0 < lv; l0 += 4u) {
         const uint32_t l = l0 + g;
-        BinsEval e{ 0, 0.0, 0u, 0u, false };
         uint32_t first = 0, nch = 0, own = 0;
         if (l < lv) {
             const uint4 ma = __ldg(&meta[M.chain[l]]);
             first = ma.x;
             nch = (uint32_t)__popc(topo_mask(ma.y));
             own = M.chain[l + 1u] - first;
-            if (sub < nch) {
-                e = ev(first + sub);
-            }
         }
-        const uint32_t own_exp = __ballot_sync(0xFFFFFFFFu, l < lv && sub == own && e.status == 1);
+        const BinsEval e = ev(first + sub, sub < nch);
+        const uint32_t own_exp = __ballot_sync(0xFFFFFFFFu, l < lv && sub == own && e.expand);
         // a level is visited when every own child above it was expanded
         bool visit = l < lv;
         for (uint32_t q = 0; q < g; ++q) {
@@ -250,14 +242,14 @@ __device__ int32_t bins_search(const BinsMem& M, const uint4* __restrict__ meta,
         seen += act ? 1u : 0u;
         any = any || (act && e.cand);
         const bool mine_exp = ((own_exp >> (8u * g)) & 0xFFu) != 0u;
-        const bool push = act && e.status == 1 && sub != own;
+        const bool push = act && e.expand && sub != own;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, push);
-        const uint32_t exp_all = __ballot_sync(0xFFFFFFFFu, act && e.status == 1);
+        const uint32_t exp_all = __ballot_sync(0xFFFFFFFFu, act && e.expand);
         if (push) {
             M.stack[top + (uint32_t)__popc(m & ((1u << lane) - 1u))] = make_uint2(e.first, (l * 8u + sub) | (e.nch << 16));
         }
         top += (uint32_t)__popc(m);
-        if (act && e.status == 2) {
+        if (act && e.cand) {
             M.bin[l * 8u + sub] = e.w;
         }
         if (visit && sub == 0u) {

@@ -653,9 +653,9 @@ struct BinsArgs {
     unsigned long long* touched;
 };
 
-// Whether an inner node at (dx, dy, dz) from the source is expanded, accepted
-// or discarded, by evaluate's own operations (for the rare nodes whose test
-// is too close for the squared form).
+// Whether a node at (dx, dy, dz) from the source is expanded, accepted or
+// discarded, by evaluate's own operations (for the rare nodes whose test is
+// too close for the squared form).
 __device__ __noinline__ int exact_status(double dx, double dy, double dz, double md, double theta, bool leaf) {
     const double d = rl_hypot3(dx, dy, dz);
     if (d == 0.0) {
@@ -680,58 +680,58 @@ struct Bins64 {
     const uint4* __restrict__ meta;
     const double* tab;  // 2^(j/64) in shared memory
     double sx, sy, sz;
+    double scale;
     double to_k;  // -64 / (ln 2 sigma^2)
     float theta2;
+    float far2;   // squared distances from here on weigh less than exp(-699): taken as 0
     uint32_t source, num_nodes;
 
-    __device__ __forceinline__ BinsEval operator()(uint32_t nd) const {
-        BinsEval e{ ST_DISCARD, 0.0, 0u, 0u, false };
-        if (nd >= num_nodes) {
-            return e;
-        }
+    __device__ __forceinline__ BinsEval operator()(uint32_t nd, bool act) const {
+        act = act && nd < num_nodes;
+        nd = act ? nd : 0u;
         const uint4 mm = __ldg(&meta[nd]);
         const double4 rr = ldg4(&rec[nd]);
         const bool leaf = topo_leaf(mm.y);
+        const bool self = leaf && mm.x == source;
+        BinsEval e;
+        e.first = mm.x;
+        e.nch = (uint32_t)__popc(topo_mask(mm.y));
         if constexpr (!SQUARED) {
-            const Eval ev = evaluate(rr, make_uint2(mm.x, mm.y), __ldg(&S.maxdim[nd]), sx, sy, sz, source, W.theta, S.mu, W.scale, false, S.kernel);
-            e.status = ev.status;
+            Eval ev{ ST_DISCARD, 0.0 };
+            if (act) {
+                ev = evaluate(rr, make_uint2(mm.x, mm.y), __ldg(&S.maxdim[nd]), sx, sy, sz, source, W.theta, S.mu, scale, false, S.kernel);
+            }
             e.w = ev.w;
-            e.cand = ev.status == ST_ACCEPT && !(leaf && mm.x == source);
+            e.expand = ev.status == ST_EXPAND;
+            e.cand = ev.status == ST_ACCEPT && !self;
         } else {
             const uint32_t cnt = rcount(rr);
-            if (cnt == 0u || (leaf && mm.x == source)) {
-                return e;  // the source itself weighs 0: as good as discarded
-            }
+            bool live = act && cnt != 0u && !self;  // the source itself weighs 0: as good as discarded
             const double dx = rr.x - sx, dy = rr.y - sy, dz = rr.z - sz;
             const double d2 = __fma_rn(dx, dx, __fma_rn(dy, dy, dz * dz));
             const float md = __uint_as_float(mm.w);
-            const float m2 = md * md, t2 = theta2 * (float)d2;
-            int status = leaf || m2 < t2 ? ST_ACCEPT : ST_EXPAND;
-            if ((!leaf && fabsf(m2 - t2) <= 2e-6f * m2) || d2 < 1e-200) {
-                status = exact_status(dx, dy, dz, __ldg(&S.maxdim[nd]), W.theta, leaf);
+            const float d2f = (float)d2;
+            const float m2 = md * md, t2 = theta2 * d2f;
+            bool accept = leaf || m2 < t2;
+            if (live && ((!leaf && fabsf(m2 - t2) <= 2e-6f * m2) || d2f < 1e-30f)) {
+                const int status = exact_status(dx, dy, dz, __ldg(&S.maxdim[nd]), W.theta, leaf);
+                live = status != ST_DISCARD;
+                accept = status == ST_ACCEPT;
             }
-            e.status = status;
-            if (status == ST_ACCEPT) {
-                // 2^(k/64) e^s with k the nearest integer (1.5 x 2^52 rounds it), |s| < 0.0055:
-                // Tang's reduction as in rl_exp, to 4e-14 of the value
-                const double km = __fma_rn(d2, to_k, 6755399441055744.0);
-                const double kd = km - 6755399441055744.0;
-                const double x = d2 * W.scale;
-                const double s = __fma_rn(kd, -0.010830424696249145, x);  // ln 2 / 64
-                double q = __fma_rn(s, 1.0 / 24.0, 1.0 / 6.0);
-                q = __fma_rn(q, s, 0.5);
-                q = __fma_rn(q, s, 1.0);
-                const int k = __double2loint(km);
-                const double t = tab[k & 63];
-                const double t2m = __hiloint2double(__double2hiint(t) + ((k >> 6) << 20), __double2loint(t));
-                const double w = __fma_rn(t2m * s, q, t2m);
-                e.w = x < -700.0 ? 0.0 : w * (double)cnt;
-                e.cand = true;
-            }
-        }
-        if (e.status == ST_EXPAND) {
-            e.first = mm.x;
-            e.nch = (uint32_t)__popc(topo_mask(mm.y));
+            // 2^(k/64) e^s with k the nearest integer (1.5 x 2^52 rounds it), |s| < 0.0055:
+            // Tang's reduction as in rl_exp, to 4e-14 of the value
+            const double km = __fma_rn(d2, to_k, 6755399441055744.0);
+            const double s = __fma_rn(km - 6755399441055744.0, -0.010830424696249145, d2 * scale);  // ln 2 / 64
+            double q = __fma_rn(s, 1.0 / 24.0, 1.0 / 6.0);
+            q = __fma_rn(q, s, 0.5);
+            q = __fma_rn(q, s, 1.0);
+            const int k = __double2loint(km);
+            const double t = tab[k & 63];
+            const double t2m = __hiloint2double(__double2hiint(t) + ((k >> 6) << 20), __double2loint(t));
+            const double w = __fma_rn(t2m * s, q, t2m) * (double)cnt;
+            e.cand = live && accept;
+            e.w = e.cand && d2f <= far2 ? w : 0.0;
+            e.expand = live && !accept;
         }
         return e;
     }
@@ -747,7 +747,7 @@ constexpr double kBinsMargin64 = 2e-11;
 constexpr double kBinsTiny64 = 1e-250;
 
 template <int WPB, bool SQUARED>
-__global__ void __launch_bounds__(WPB * 32, SQUARED ? 20 / WPB : 16 / WPB) k_search_bins(BinsArgs A) {
+__global__ void __launch_bounds__(WPB * 32, SQUARED ? 24 / WPB : 16 / WPB) k_search_bins(BinsArgs A) {
     extern __shared__ __align__(16) unsigned char smem_bins[];
     double* tab = reinterpret_cast<double*>(smem_bins);
     for (uint32_t i = threadIdx.x; i < 64u; i += WPB * 32) {
@@ -782,8 +782,9 @@ __global__ void __launch_bounds__(WPB * 32, SQUARED ? 20 / WPB : 16 / WPB) k_sea
         if (!N.root_leaf) {
             const uint32_t source = S.list_src[idx];
             const uint32_t j = S.list_j[idx];
-            const Bins64<SQUARED> ev{ S, W, S.rec, S.meta, tab, S.px[source], S.py[source], S.pz[source], W.scale * 92.332482616893656768, (float)(W.theta * W.theta),
-                                      source, S.num_nodes };
+            const Bins64<SQUARED> ev{ S, W, S.rec, S.meta, tab, S.px[source], S.py[source], S.pz[source], W.scale, W.scale * 92.332482616893656768,
+                                      (float)(W.theta * W.theta),
+                                      (float)fmin(-699.0 / W.scale, 3e38), source, S.num_nodes };
             result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny64, touched, ev,
                                  [&](double total, uint32_t depth) { return pick_threshold(total, W.seed, S.step, source - W.first, j, depth); },
                                  [&](double total, uint32_t visited) { return total * (kBinsMargin64 + (double)visited * 4.5e-16); });

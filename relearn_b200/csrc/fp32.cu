@@ -1323,8 +1323,53 @@ struct BinsArgs32 {
 constexpr double kBinsMargin32 = 3.3e-7;
 constexpr double kBinsTiny32 = 1e-30;
 
-template <int WPB>
-__global__ void __launch_bounds__(WPB * 32, 32 / WPB) k_search_bins32(BinsArgs32 A) {
+// eval32's operations without its branches (the Gaussian kernel): the same
+// status and the same bits of the weight.
+template <bool GAUSS>
+struct Bins32 {
+    const Search32& S;
+    const Net32& W;
+    const uint4* __restrict__ rec;
+    const uint4* __restrict__ meta;
+    QPos sp;
+    float quantum, theta, mu, inv_sigma2;
+    uint32_t source, num_nodes;
+
+    __device__ __forceinline__ BinsEval operator()(uint32_t nd, bool act) const {
+        act = act && nd < num_nodes;
+        nd = act ? nd : 0u;
+        const uint4 mm = __ldg(&meta[nd]);
+        const uint4 rr = __ldg(&rec[nd]);
+        const bool leaf = topo_leaf(mm.y);
+        const bool self = leaf && mm.x == source;
+        BinsEval e;
+        e.first = mm.x;
+        e.nch = (uint32_t)__popc(topo_mask(mm.y));
+        if constexpr (!GAUSS) {
+            E32 v{ S_DISCARD, 0.0f };
+            if (act) {
+                v = eval32(rr, mtopo(mm), mmaxdim(mm), sp, source, S, W, false);
+            }
+            e.w = (double)v.w;
+            e.expand = v.status == S_EXPAND;
+            e.cand = v.status == S_ACCEPT && !self;
+        } else {
+            const float dx = qdiff(rr.x, sp.x, quantum), dy = qdiff(rr.y, sp.y, quantum), dz = qdiff(rr.z, sp.z, quantum);
+            const float d = dist32(dx, dy, dz);
+            const bool live = act && rr.w != 0u && d != 0.0f;
+            const bool accept = leaf || mmaxdim(mm) < theta * d;
+            const float dm = d - mu;
+            const float w = __expf(-(dm * dm) * inv_sigma2) * (float)rr.w;
+            e.cand = live && accept && !self;
+            e.w = (double)(e.cand ? w : 0.0f);
+            e.expand = live && !accept;
+        }
+        return e;
+    }
+};
+
+template <int WPB, bool GAUSS>
+__global__ void __launch_bounds__(WPB * 32, 24 / WPB) k_search_bins32(BinsArgs32 A) {
     extern __shared__ __align__(16) unsigned char smem_bins[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -1357,23 +1402,7 @@ __global__ void __launch_bounds__(WPB * 32, 32 / WPB) k_search_bins32(BinsArgs32
             const QFrame& F = N.frame;
             const QPos sp{ quantize(S.px[source], F.origin[0], F.inv_quantum), quantize(S.py[source], F.origin[1], F.inv_quantum),
                            quantize(S.pz[source], F.origin[2], F.inv_quantum) };
-            auto ev = [&](uint32_t nd) {
-                BinsEval r{ S_DISCARD, 0.0, 0u, 0u, false };
-                if (nd >= S.num_nodes) {
-                    return r;
-                }
-                const uint4 mm = __ldg(&S.meta[nd]);
-                const E32 e = eval32(__ldg(&S.rec[nd]), mtopo(mm), mmaxdim(mm), sp, source, S, W, false);
-                r.status = e.status;
-                if (e.status == S_ACCEPT) {
-                    r.w = (double)e.w;
-                    r.cand = !(topo_leaf(mm.y) && mm.x == source);
-                } else if (e.status == S_EXPAND) {
-                    r.first = mm.x;
-                    r.nch = (uint32_t)__popc(topo_mask(mm.y));
-                }
-                return r;
-            };
+            const Bins32<GAUSS> ev{ S, W, S.rec, S.meta, sp, W.quantum, W.theta, S.mu, W.inv_sigma2, source, S.num_nodes };
             result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny32, touched, ev,
                                  [&](double total, uint32_t depth) {
                                      const u32x4 w = draw(W.seed, S.step, source - W.first, j, STREAM_BH_PICK, depth);  // as threshold32
@@ -1809,7 +1838,7 @@ void launch_search_wide_f32(Ctx& c, const uint32_t (&warps)[2], uint32_t segs0, 
     B.tasks = S.tasks.p;
     B.counts = S.w_counts.p;
     {
-        auto kern = &k_search_bins32<WPB>;
+        auto kern = c.kernel.type == RL_KERNEL_GAUSSIAN ? &k_search_bins32<WPB, true> : &k_search_bins32<WPB, false>;
         const size_t smem = WPB * bins_warp_bytes(B.levels);
         RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;

@@ -279,10 +279,15 @@ struct ActDesc {
 };
 
 // Launch shape of the Barnes-Hut search kernels.
+// Without tuning: one search per warp by bins (packet 0), the fastest form in
+// every density class measured (1M neurons, every neuron searching: 32.7 ms
+// against 72.3 ms for packets of 32 in FP64, 25.3 against 33.4 ms in FP32;
+// 20,000 searches: 0.80 against 47 ms; 52,000 neurons, 260 searches: 0.11
+// against 23 ms).
 struct SearchVariant {
-    int warps = 2;    // warps per block
-    int packet = 32;  // lanes (sources) that walk the descent from the root together
-    int cap = 1;      // 1: registers capped at 64 for more resident warps
+    int warps = 4;    // warps per block
+    int packet = 0;   // lanes (sources) that walk the descent from the root together; 0: one search per warp
+    int cap = 0;      // 1: registers capped at 64 for more resident warps
     int hot = 0;      // > 0: persistent form, one block of 32 warps per SM with up
                       // to `hot` top octree nodes in shared memory
 };
