@@ -1164,41 +1164,14 @@ rl_status rl_add_edges(void* ctx, uint64_t m, const uint32_t* target, const uint
 rl_status rl_get_edges(void* ctx, uint32_t* target, uint32_t* source, int32_t* weight, uint64_t capacity, uint64_t* count) {
     return rl::guarded(ctx, [&](Ctx& c) {
         rl::rebuild_graph(c);
-        const uint64_t m = c.graph.num_edges;
-        std::vector<uint32_t> off(c.n + 1), s(m);
-        std::vector<int32_t> w(m);
-        RL_CUDA_TRY(cudaMemcpyAsync(off.data(), c.graph.offsets.p, (c.n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
-        if (m) {
-            RL_CUDA_TRY(cudaMemcpyAsync(s.data(), c.graph.src.p, m * 4, cudaMemcpyDeviceToHost, c.stream));
-            RL_CUDA_TRY(cudaMemcpyAsync(w.data(), c.graph.weight.p, m * 4, cudaMemcpyDeviceToHost, c.stream));
-        }
-        RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
-        // aggregate (target, source) pairs, drop zero weights (NetworkGraph::add_edge)
-        uint64_t k = 0;
-        std::vector<std::pair<uint32_t, int32_t>> row;
-        for (uint32_t t = 0; t < c.n; ++t) {
-            row.clear();
-            for (uint32_t e = off[t]; e < off[t + 1]; ++e) {
-                row.emplace_back(s[e], w[e]);
-            }
-            std::sort(row.begin(), row.end());
-            for (size_t a = 0; a < row.size();) {
-                size_t b = a;
-                int64_t sum = 0;
-                while (b < row.size() && row[b].first == row[a].first) {
-                    sum += row[b].second;
-                    ++b;
-                }
-                if (sum != 0) {
-                    if (k < capacity) {
-                        if (target) target[k] = t;
-                        if (source) source[k] = row[a].first;
-                        if (weight) weight[k] = (int32_t)sum;
-                    }
-                    ++k;
-                }
-                a = b;
-            }
+        const bool fill = capacity > 0 && (target || source || weight);
+        const uint64_t k = rl::aggregate_edges(c, !fill);
+        const uint64_t out = fill ? std::min(k, capacity) : 0;
+        if (out) {
+            if (target) rl::download(target, c.graph.m_tgt, out, c.stream);
+            if (source) rl::download(source, c.graph.m_src, out, c.stream);
+            if (weight) rl::download(weight, c.graph.m_w, out, c.stream);
+            RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
         }
         if (count) *count = k;
     });

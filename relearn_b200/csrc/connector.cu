@@ -514,6 +514,43 @@ void sort_new(Ctx& c, uint64_t* key, uint32_t* val, uint64_t m, int bits) {
     radix_sort_u64(key, val, m, bits, c.prim, c.stream);
 }
 
+// Runs of equal (target, source) pairs of the sorted list (NetworkGraph::add_edge
+// aggregates them): the run's first entry receives the summed weight, and
+// keep[e] is 1 for the first entry of a run whose sum is not 0.
+__global__ void k_edge_runs(uint64_t m, const uint32_t* __restrict__ t, const uint32_t* __restrict__ src, const int32_t* __restrict__ w,
+                            uint32_t* __restrict__ keep, int32_t* __restrict__ sum_out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m) {
+        return;
+    }
+    const uint32_t tt = t[e], ss = src[e];
+    uint32_t k = 0;
+    if (e == 0 || t[e - 1] != tt || src[e - 1] != ss) {
+        int64_t sum = w[e];
+        for (uint64_t f = e + 1; f < m && t[f] == tt && src[f] == ss; ++f) {
+            sum += w[f];
+        }
+        sum_out[e] = (int32_t)sum;
+        k = sum != 0 ? 1u : 0u;
+    }
+    keep[e] = k;
+}
+
+// Entry e of the list is the pos[e]-th kept one where the positions step.
+__global__ void k_edge_out(uint64_t m, uint64_t kept, const uint32_t* __restrict__ pos, const uint32_t* __restrict__ t, const uint32_t* __restrict__ src,
+                           const int32_t* __restrict__ sum, uint32_t* __restrict__ t_out, uint32_t* __restrict__ s_out, int32_t* __restrict__ w_out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m) {
+        return;
+    }
+    const uint32_t p = pos[e];
+    if ((e + 1 < m ? pos[e + 1] : (uint32_t)kept) != p) {
+        t_out[p] = t[e];
+        s_out[p] = src[e];
+        w_out[p] = sum[e];
+    }
+}
+
 }  // namespace
 
 // Merges the new synapses into the sorted list and the out-CSR, drops the
@@ -622,6 +659,34 @@ void rebuild_graph(Ctx& c) {
     RL_LAUNCH_CHECK();
     k_row_offsets<<<blocks_for(m + 1, 256), 256, 0, st>>>(m, G.src.p, G.out_perm.p, n, G.out_off.p);
     RL_LAUNCH_CHECK();
+}
+
+// The aggregated synapse list (equal pairs summed, zero sums dropped, sorted
+// by target and source) in the rebuild's working arrays m_tgt, m_src, m_w;
+// returns its length.  The list is sorted already, so it takes one pass over
+// it, a scan and a compaction on the device (500,000 synapses: copying the raw
+// list out and sorting its rows on the host took 3 ms per call).
+uint64_t aggregate_edges(Ctx& c, bool count_only) {
+    Graph& G = c.graph;
+    const uint64_t m = G.num_edges;
+    if (m == 0) {
+        return 0;
+    }
+    cudaStream_t st = c.stream;
+    G.m_pos.fit(m);
+    G.m_out.fit(m);
+    int32_t* sum = reinterpret_cast<int32_t*>(G.m_out.p);
+    k_edge_runs<<<blocks_for(m, 256), 256, 0, st>>>(m, G.tgt.p, G.src.p, G.weight.p, G.m_pos.p, sum);
+    RL_LAUNCH_CHECK();
+    const uint64_t kept = exclusive_scan_u32(G.m_pos.p, G.m_pos.p, m, c.prim, st);
+    if (!count_only && kept) {
+        G.m_tgt.fit(kept);
+        G.m_src.fit(kept);
+        G.m_w.fit(kept);
+        k_edge_out<<<blocks_for(m, 256), 256, 0, st>>>(m, kept, G.m_pos.p, G.tgt.p, G.src.p, sum, G.m_tgt.p, G.m_src.p, G.m_w.p);
+        RL_LAUNCH_CHECK();
+    }
+    return kept;
 }
 
 uint64_t run_deletion(Ctx& c, uint32_t step, int type) {

@@ -464,6 +464,7 @@ void run_search(Ctx& c, uint32_t step);  // fills search.req_* (requests in (sou
 uint64_t run_connector(Ctx& c, uint32_t step, bool bind_axons = true);
 void bind_axons_host(Ctx& c, uint64_t m, const uint32_t* src);  // one vacant axon per listed source
 void rebuild_graph(Ctx& c);                     // merge new edges into the CSR
+uint64_t aggregate_edges(Ctx& c, bool count_only);  // the list rl_get_edges returns, in graph.m_tgt, m_src, m_w
 uint64_t run_deletion(Ctx& c, uint32_t step, int type);  // delete to_delete[] synapses per neuron for one element type
 void add_edges_host(Ctx& c, uint64_t m, const uint32_t* t, const uint32_t* s, const int32_t* w);
 
