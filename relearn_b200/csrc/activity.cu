@@ -44,6 +44,7 @@ struct ActArgs {
     double syn0;  // the synaptic input without in-edges: 0.0 + 0.0 * conductance
     uint32_t h_model, h_calcium;
     double a, ab, c, d, v_spike, k1, k2, k3, scale_m;
+    uint32_t spike_hi;  // high word of v_spike where izhikevich_frozen may compare it alone, else 0
     double beta, tau_inv, scale_c;
     double eta[3];
     const NetInfo* nets;
@@ -104,16 +105,16 @@ __device__ __forceinline__ double growth_curve_pre(double current, double eta, i
     return rl_fma(2.0, rl_exp(-prod), -1.0);  // (2 e) - 1, as in growth_curve
 }
 
-// growth_curve_pre without branches (rl_exp_flat; the eta == epsilon case
-// selected), for the software-pipelined block kernel.
+// growth_curve_pre without branches (the eta == epsilon case selected), for
+// the software-pipelined block kernel.  Equality with eta is compared on the
+// bits (a calcium after its step is never -0, and NaN equals nothing).
 __device__ __forceinline__ double growth_curve_flat(double current, double eta, int flat, double xi, double zeta, double zeta_inv) {
     const double diff = current - xi;
     const double q0 = diff * zeta_inv;
     const double r = rl_fma(-zeta, q0, diff);
     const double quot = rl_fma(r, zeta_inv, q0);
-    const double prod = quot * quot;
-    const double g = rl_fma(2.0, rl_exp_flat_nonpos(-prod), -1.0);
-    return flat ? (current == eta ? 0.0 : -1.0) : g;
+    const double g = rl_two_exp_minus_one(quot * quot);
+    return flat ? (__double_as_longlong(current) == __double_as_longlong(eta) ? 0.0 : -1.0) : g;
 }
 
 // The network of neuron i: draws are keyed on the network's seed and the
@@ -260,7 +261,10 @@ __device__ __forceinline__ double growth_step(const ActArgs& A, int t, double ca
 // no branch (a branch ends the stretch of code the compiler schedules
 // together), and a substep costs one select (the u of a first crossing) on
 // top of the model's arithmetic.
-template <int H>
+// TOP: v_spike is positive with a low word of 0, so x >= v_spike for x up to
+// +infinity is one unsigned comparison of the high words (NaN lies above it),
+// off the FP64 pipe that bounds the block kernel.
+template <int H, bool TOP>
 __device__ __forceinline__ uint8_t izhikevich_frozen(const ActArgs& A, double input, double& x, double& u) {
     double xv = x;
     double uv = u;
@@ -272,7 +276,8 @@ __device__ __forceinline__ uint8_t izhikevich_frozen(const ActArgs& A, double in
         const double u_inc = (A.ab * xv) - (A.a * uv);
         xv = xv + x_inc * A.scale_m;
         uv = uv + u_inc * A.scale_m;
-        const bool first = !done && xv >= A.v_spike;
+        const bool top = TOP ? (uint32_t)__double2hiint(xv) - A.spike_hi <= 0x7FF00000u - A.spike_hi : xv >= A.v_spike;
+        const bool first = !done && top;
         u_cross = first ? uv : u_cross;
         done = done || first;
     }
@@ -315,15 +320,15 @@ __device__ __forceinline__ void calcium_growth_flat(const ActArgs& A, uint8_t sp
 // order, so the bits are too.  zs[k * stride] is step k's standard normal
 // draw; `input` receives the last step's input, f and f_before the last two
 // spike flags.
-template <int H, bool MULTI>
+template <int H, bool MULTI, bool TOP>
 __device__ __forceinline__ void izhikevich_chunk(const ActArgs& A, const double* zs, uint32_t stride, uint32_t m, const Nu& nu, double& xv,
                                                  double& uv, double& ca, double& d0, double& d1, double& d2, double& input, uint8_t& f,
                                                  uint8_t& f_before) {
     double in_k = A.syn0 + (A.noise_mean + A.noise_stddev * zs[0]);
-    uint8_t sp = izhikevich_frozen<H>(A, in_k, xv, uv);
+    uint8_t sp = izhikevich_frozen<H, TOP>(A, in_k, xv, uv);
     for (uint32_t k = 0; k + 1 < m; ++k) {
         const double in_n = A.syn0 + (A.noise_mean + A.noise_stddev * zs[(k + 1) * stride]);
-        const uint8_t sp_n = izhikevich_frozen<H>(A, in_n, xv, uv);
+        const uint8_t sp_n = izhikevich_frozen<H, TOP>(A, in_n, xv, uv);
         calcium_growth_flat<H, MULTI>(A, sp, nu, ca, d0, d1, d2);
         f_before = f;
         f = sp;
@@ -471,7 +476,7 @@ __global__ void __launch_bounds__(BLOCK) k_activity(ActArgs A, const ActDesc* __
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     if (on[v]) {
-                        p[v] = ((double)noise_bits53(r, i[v]) + 0.5) * 1.1102230246251565404e-16;  // noise_uniform_rk's open (0, 1)
+                        p[v] = uniform_from_bits53(noise_bits53(r, i[v]));  // as noise_uniform_rk
                     }
                 }
             }
@@ -521,7 +526,7 @@ __global__ void __launch_bounds__(BLOCK) k_activity(ActArgs A, const ActDesc* __
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 in[v] = step_input(A, isum[v], z[v]);
-                sp[v] = izhikevich_frozen<H>(A, in[v], xv[v], uv[v]);
+                sp[v] = izhikevich_frozen<H, false>(A, in[v], xv[v], uv[v]);
             }
 #pragma unroll
             for (int v = 0; v < V; ++v) {
@@ -626,7 +631,7 @@ constexpr int kDrawChunk = 10;
 // k + 1's, and each hands the other the two words it needs (the same words as
 // a block per lane).  `parity` selects the shared tail-queue counter of the
 // next chunk.
-template <int BLOCK, int H, int MODEL, bool MULTI>
+template <int BLOCK, int H, int MODEL, bool MULTI, bool TOP>
 __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* __restrict__ D, uint32_t nsteps,
                                                uint8_t* __restrict__ fired_before_last, uint32_t i, bool in, uint64_t seed, uint32_t local,
                                                const Nu& nu, const uint32_t (&rk0)[10], const uint32_t (&rk1)[10], uint32_t& parity, double* s_z,
@@ -668,7 +673,7 @@ __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* 
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const bool use = on && (uint32_t)(k + h) < m;
-                const double p = ((double)b[h] + 0.5) * 1.1102230246251565404e-16;  // open (0, 1)
+                const double p = uniform_from_bits53(b[h]);  // open (0, 1)
                 const bool tail = use && normal_in_tail(p);
                 const uint32_t mask = __ballot_sync(0xFFFFFFFFu, tail);
                 uint32_t first = 0;
@@ -696,7 +701,7 @@ __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* 
         bool piped = false;
         if constexpr (MODEL == RL_MODEL_IZHIKEVICH && H > 0) {
             if (on && A.uniform_target) {
-                izhikevich_chunk<H, MULTI>(A, s_z + threadIdx.x, BLOCK, m, nu, xv, uv, ca, d0, d1, d2, input, f, f_before);
+                izhikevich_chunk<H, MULTI, TOP>(A, s_z + threadIdx.x, BLOCK, m, nu, xv, uv, ca, d0, d1, d2, input, f, f_before);
                 piped = true;
             }
         }
@@ -754,7 +759,7 @@ __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* 
 // of A.blocks, each of one network and starting at an even index of it (a
 // multiple of kNetBlock), so that the seed and growth rates are the block's
 // and every lane pair holds a neuron pair.
-template <int BLOCK, int H, int MODEL, bool MULTI>
+template <int BLOCK, int H, int MODEL, bool MULTI, bool TOP>
 __global__ void __launch_bounds__(BLOCK, (MULTI ? 640 : 768) / BLOCK) k_activity_steps(ActArgs A, const ActDesc* __restrict__ D, uint32_t nsteps,
                                                                           uint8_t* __restrict__ fired_before_last) {
     __shared__ double s_z[kDrawChunk * BLOCK];      // draw of step k0 + k of thread t at k * BLOCK + t
@@ -772,7 +777,7 @@ __global__ void __launch_bounds__(BLOCK, (MULTI ? 640 : 768) / BLOCK) k_activity
             const NetBlock B = A.blocks[b];
             const NetInfo& N = A.nets[B.net];
             const Nu nu{ { N.nu[0], N.nu[1], N.nu[2] } };
-            neuron_steps64<BLOCK, H, MODEL, true>(A, D, nsteps, fired_before_last, B.first + threadIdx.x, threadIdx.x < B.count, N.seed,
+            neuron_steps64<BLOCK, H, MODEL, true, TOP>(A, D, nsteps, fired_before_last, B.first + threadIdx.x, threadIdx.x < B.count, N.seed,
                                                   B.first - N.first + threadIdx.x, nu, A.rk0, A.rk1, parity, s_z, s_who, s_cnt);
         }
     } else {
@@ -780,7 +785,7 @@ __global__ void __launch_bounds__(BLOCK, (MULTI ? 640 : 768) / BLOCK) k_activity
         const Nu nu{ { A.nu1[0], A.nu1[1], A.nu1[2] } };
         for (uint32_t base = blockIdx.x * BLOCK; base < A.n; base += stride) {
             const uint32_t i = base + threadIdx.x;
-            neuron_steps64<BLOCK, H, MODEL, false>(A, D, nsteps, fired_before_last, i, i < A.n, A.seed1, i, nu, A.rk0, A.rk1, parity, s_z,
+            neuron_steps64<BLOCK, H, MODEL, false, TOP>(A, D, nsteps, fired_before_last, i, i < A.n, A.seed1, i, nu, A.rk0, A.rk1, parity, s_z,
                                                    s_who, s_cnt);
         }
     }
@@ -971,6 +976,11 @@ ActArgs act64_args(Ctx& c, uint32_t kstep, const uint8_t* fired_prev, uint8_t* f
     A.c = k.iz_c;
     A.d = k.iz_d;
     A.v_spike = k.iz_v_spike;
+    {
+        const uint64_t bits = as_u64(k.iz_v_spike);
+        const bool top = k.iz_v_spike > 0.0 && (uint32_t)bits == 0u && bits < 0x7FF0000000000000ull;
+        A.spike_hi = top ? (uint32_t)(bits >> 32) : 0u;
+    }
     A.k1 = k.iz_k1;
     A.k2 = k.iz_k2;
     A.k3 = k.iz_k3;
@@ -1026,13 +1036,13 @@ ActArgs act64_args(Ctx& c, uint32_t kstep, const uint8_t* fired_prev, uint8_t* f
     return A;
 }
 
-template <int BLOCK, int H, int MODEL>
+template <int BLOCK, int H, int MODEL, bool TOP = false>
 void launch_steps64_m(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_before_last) {
     if (c.multi()) {
-        launch_pdl(&k_activity_steps<BLOCK, H, MODEL, true>, c.num_net_blocks, BLOCK, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
+        launch_pdl(&k_activity_steps<BLOCK, H, MODEL, true, TOP>, c.num_net_blocks, BLOCK, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
                    fired_before_last);
     } else {
-        launch_pdl(&k_activity_steps<BLOCK, H, MODEL, false>, blocks_for(c.n, BLOCK), BLOCK, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
+        launch_pdl(&k_activity_steps<BLOCK, H, MODEL, false, TOP>, blocks_for(c.n, BLOCK), BLOCK, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
                    fired_before_last);
     }
 }
@@ -1050,7 +1060,11 @@ void launch_steps64(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_be
             launch_steps64_m<128, H, RL_MODEL_AEIF>(c, A, nsteps, fired_before_last);
             break;
         default:
-            launch_steps64_m<128, H, RL_MODEL_IZHIKEVICH>(c, A, nsteps, fired_before_last);
+            if (H > 0 && A.spike_hi != 0u) {
+                launch_steps64_m<128, H, RL_MODEL_IZHIKEVICH, true>(c, A, nsteps, fired_before_last);
+            } else {
+                launch_steps64_m<128, H, RL_MODEL_IZHIKEVICH>(c, A, nsteps, fired_before_last);
+            }
             break;
     }
 }

@@ -376,6 +376,50 @@ RL_HD double rl_exp_flat_nonpos(double x) {
     return x != x ? x : (x < -745.1332191019412 ? 0.0 : v);
 }
 
+// 2 exp(-q) - 1 for q >= 0 and NaN (the growth curve), rounded once at the
+// end: the bits of rl_fma(2.0, rl_exp(-q), -1.0), in 15 FP64 operations and
+// without conversions or comparisons in FP64.
+//   * floor(t) comes from adding 1.5 x 2^52 with rounding towards -infinity,
+//     which also leaves the integer in the low word;
+//   * k ln2/64 (high part) is exact, so one fused multiply-add subtracts it;
+//   * 2^m y is exact for m >= -1000, so 2 (2^m y) - 1 is one fused
+//     multiply-add with 2^(m+1); below that the sum rounds to -1 whatever the
+//     factor, so m is held at -1000;
+//   * from q = 740 on exp(-q) is below 1e-321 and the result -1 (one integer
+//     comparison of the high word, which leaves NaN to the arithmetic).
+RL_HD double rl_two_exp_minus_one(double q) {
+#if defined(__CUDA_ARCH__)
+    const double x = -q;
+    const double km = __dadd_rd(x * RL_EXPC(5) + 0.5, 6755399441055744.0);
+    const double kd = km - 6755399441055744.0;
+    const int ki = __double2loint(km);
+    const uint32_t qh = (uint32_t)__double2hiint(q);
+#else
+    const double x = q >= 740.0 ? -740.0 : -q;  // keeps the host's conversion defined
+    const double kd = x != x ? x : floor(x * RL_EXPC(5) + 0.5);
+    const int ki = x != x ? 0 : (int)kd;
+    const uint32_t qh = (uint32_t)(as_u64(q) >> 32);
+#endif
+    const double r = rl_fma(-kd, RL_EXPC(7), rl_fma(-kd, RL_EXPC(6), x));
+    const int j = ki & 63;
+    const int m = ki >> 6;
+    double p = rl_fma(RL_EXPC(0), r, RL_EXPC(1));
+    p = rl_fma(p, r, RL_EXPC(2));
+    p = rl_fma(p, r, RL_EXPC(3));
+    p = rl_fma(p, r, RL_EXPC(4));
+    p = rl_fma(r * r, p, r);
+#if defined(__CUDA_ARCH__)
+    const double2 t = __ldg(&rl_exp_table_dev[j]);
+    const double t_hi = t.x, t_lo = t.y;
+#else
+    const double t_hi = rl_exp_table_host[j][0], t_lo = rl_exp_table_host[j][1];
+#endif
+    const double y = t_hi + rl_fma(t_hi, p, t_lo);
+    const int mm = m < -1000 ? -1000 : m;
+    const double g = rl_fma(y, as_f64((uint64_t)(uint32_t)(mm + 1024) << 52), -1.0);
+    return qh - 0x40872000u <= 0x7FF00000u - 0x40872000u ? -1.0 : g;
+}
+
 // log(x) for finite x > 0 (normal range): x = m 2^e with m in
 // [sqrt(2)/2, sqrt(2)), log(m) = 2 atanh(s), s = (m-1)/(m+1), odd series in s.
 RL_HD double rl_log(double x) {
@@ -526,8 +570,10 @@ RL_HD double next_up_eps(double total) {
 // the central rational function for |p - 0.5| <= 0.425 and the tails.  A
 // kernel that draws for many neurons runs the tail piece for the few that need
 // it together (it holds a log, a square root and two divisions).
+// (p - 0.5 is never NaN here, so its distance from 0 is compared as an
+// integer, off the FP64 pipe.)
 RL_HD bool normal_in_tail(double p) {
-    return !(fabs(p - 0.5) <= 0.425);
+    return (as_u64(p - 0.5) & 0x7FFFFFFFFFFFFFFFull) > 0x3FDB333333333333ull;  // 0.425
 }
 
 // The central piece's coefficients, highest power first (numerator, then
@@ -630,15 +676,27 @@ RL_HD uint64_t noise_bits53(const u32x4& r, uint32_t neuron) {
     return (neuron & 1u) ? (((uint64_t)r.z << 21) | (uint64_t)(r.w >> 11)) : (((uint64_t)r.x << 21) | (uint64_t)(r.y >> 11));
 }
 
+// (b + 0.5) 2^-53 for 53 random bits b, as ((double)b + 0.5) * 2^-53 rounds
+// it, without converting an integer: for b < 2^52 the value (2b + 1) 2^-54 is
+// exact, and 0.5 + b 2^-53 (b as the mantissa) minus (0.5 - 2^-54) gives it;
+// from 2^52 on b + 0.5 is a tie that rounds to even, b + (b odd), which is
+// exact times 2^-53.
+RL_HD double uniform_from_bits53(uint64_t b) {
+    const bool high = (b >> 52) != 0;
+    const uint64_t even = b + (high ? b & 1u : 0u);
+    const double base = as_f64(0x3FE0000000000000ull + (high ? even - (1ull << 52) : even));
+    return base - (high ? 0.0 : as_f64(0x3FDFFFFFFFFFFFFFull));
+}
+
 // The open-interval uniform of a neuron's background draw.
 RL_HD double noise_uniform(uint64_t seed, uint32_t step, uint32_t neuron) {
     const u32x4 r = noise_block(seed, step, neuron);
-    return ((double)noise_bits53(r, neuron) + 0.5) * 1.1102230246251565404e-16;  // open (0, 1)
+    return uniform_from_bits53(noise_bits53(r, neuron));  // open (0, 1)
 }
 
 RL_HD double noise_uniform_rk(const uint32_t* rk0, const uint32_t* rk1, uint32_t step, uint32_t neuron) {
     const u32x4 r = noise_block_rk(rk0, rk1, step, neuron);
-    return ((double)noise_bits53(r, neuron) + 0.5) * 1.1102230246251565404e-16;  // open (0, 1)
+    return uniform_from_bits53(noise_bits53(r, neuron));  // open (0, 1)
 }
 
 RL_HD double background_normal(uint64_t seed, uint32_t step, uint32_t neuron, double mean, double stddev) {
