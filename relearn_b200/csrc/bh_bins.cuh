@@ -23,6 +23,8 @@
 //
 #pragma once
 
+#include <type_traits>
+
 #include "bh_wide.cuh"
 
 namespace rl {
@@ -80,36 +82,51 @@ __device__ __forceinline__ BinsMem bins_mem(unsigned char* p, uint32_t levels) {
 
 // Empties the stack of `top` entries into the bins; false if it would
 // overflow or the walk visits more nodes than there are (the ordered form
-// reports that).
+// reports that).  A pass takes the evaluator's kEntries entries per group.
 template <class Ev>
 __device__ __forceinline__ bool bins_drain(const BinsMem& M, uint32_t top, uint32_t num_nodes, uint32_t& touched, bool& any, Ev&& ev) {
+    constexpr uint32_t P = std::remove_reference_t<Ev>::kEntries;
     const uint32_t lane = threadIdx.x & 31u, g = lane >> 3, sub = lane & 7u;
     const uint32_t below = (1u << lane) - 1u;
     double* mine = M.bin + g * M.nb;
     uint32_t guard = num_nodes;
     while (top > 0u) {
-        const uint2 s = M.stack[g < top ? top - 1u - g : 0u];
-        const bool act = g < top && sub < (s.y >> 16);
-        const BinsEval e = ev(s.x + sub, act);
-        touched += act ? 1u : 0u;
-        any = any || e.cand;
-        double v = e.w;
-        v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-        v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-        v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
-        const uint32_t bin = s.y & 0xFFFFu;
-        if (sub == 0u && g < top) {
-            mine[bin] += v;
+        uint2 s[P];
+        BinsEval e[P];
+#pragma unroll
+        for (uint32_t q = 0; q < P; ++q) {
+            const uint32_t at = g + 4u * q;
+            s[q] = M.stack[at < top ? top - 1u - at : 0u];
+            const bool act = at < top && sub < (s[q].y >> 16);
+            e[q] = ev(s[q].x + sub, act);
+            touched += act ? 1u : 0u;
+            any = any || e[q].cand;
         }
-        top -= top < 4u ? top : 4u;
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, e.expand);
-        const uint32_t at = top + (uint32_t)__popc(m & below);
-        top += (uint32_t)__popc(m);
-        if (top > M.cap || guard-- == 0u) {
+#pragma unroll
+        for (uint32_t q = 0; q < P; ++q) {
+            double v = e[q].w;
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 4);
+            if (sub == 0u && g + 4u * q < top) {
+                mine[s[q].y & 0xFFFFu] += v;
+            }
+        }
+        top -= top < 4u * P ? top : 4u * P;
+#pragma unroll
+        for (uint32_t q = 0; q < P; ++q) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, e[q].expand);
+            const uint32_t at = top + (uint32_t)__popc(m & below);
+            top += (uint32_t)__popc(m);
+            if (top > M.cap) {
+                return false;
+            }
+            if (e[q].expand) {
+                M.stack[at] = make_uint2(e[q].first, (s[q].y & 0xFFFFu) | (e[q].nch << 16));
+            }
+        }
+        if (guard-- == 0u) {
             return false;
-        }
-        if (e.expand) {
-            M.stack[at] = make_uint2(e.first, bin | (e.nch << 16));
         }
         __syncwarp();
     }

@@ -674,6 +674,9 @@ __device__ __noinline__ int exact_status(double dx, double dy, double dz, double
 // counts (kBinsMargin64).  Otherwise evaluate itself.
 template <bool SQUARED>
 struct Bins64 {
+    // two entries per pass cost more registers than they hide latency (1M
+    // neurons, every neuron searching: 32.3 ms with one, 34.4 with two)
+    static constexpr uint32_t kEntries = 1;
     const SearchArgs& S;
     const WarpNet& W;
     const double4* __restrict__ rec;
@@ -690,7 +693,7 @@ struct Bins64 {
         act = act && nd < num_nodes;
         nd = act ? nd : 0u;
         const uint4 mm = __ldg(&meta[nd]);
-        const double4 rr = ldg4(&rec[nd]);
+        const double4 rr = ldg4_wide(&rec[nd]);
         const bool leaf = topo_leaf(mm.y);
         const bool self = leaf && mm.x == source;
         BinsEval e;
