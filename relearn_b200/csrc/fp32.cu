@@ -604,6 +604,193 @@ __global__ void __launch_bounds__(BLOCK) k_activity_f32_steps(Act32 A, const Act
     }
 }
 
+// Two FP32 values in one 64-bit register pair; each operation rounds both
+// halves as the scalar instruction does (fma.rn.f32x2 and its kin issue once
+// for two lanes' worth of arithmetic).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// A pair that stays in registers: the compiler would otherwise build a pair of
+// constants anew at every use (two moves each, on the pipe that bounds the
+// block kernel).
+__device__ __forceinline__ F2 f2_keep(float a, float b) {
+    F2 r = f2(a, b);
+    asm volatile("" : "+l"(r.v));
+    return r;
+}
+
+// The block of steps of an Izhikevich network without synapses with a neuron
+// pair per thread (i, i + 1 of the context; `local` even, so their draws of a
+// step are one Philox block): neuron_steps_f32's operations on both neurons,
+// two to an instruction where they are FP32.  The block kernel is bound by
+// instruction issue, and a pair issues 40 % fewer instructions than two
+// neurons on two threads.  in[v] is false for the missing half of a pair; a
+// neuron that is not enabled is computed along and keeps its state.
+template <int H>
+__device__ __forceinline__ void pair_steps_f32(const Act32& A, uint32_t step0, uint32_t nsteps, uint8_t* __restrict__ fired_before_last, uint32_t i,
+                                               const bool (&in)[2], uint32_t local, const float (&nu)[3], const uint32_t (&rk0)[10],
+                                               const uint32_t (&rk1)[10]) {
+    float xs[2], us[2], ds[3][2], xi[3][2], iz[3][2];
+    double ca[2];
+    bool en[2], f[2], f_before[2];
+    uint32_t flat[2];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        en[v] = in[v] && A.enabled[i + v] != 0;
+        f[v] = in[v] && A.fired_prev[i + v] != 0;
+        f_before[v] = f[v];
+        xs[v] = in[v] ? A.x[i + v] : 0.0f;
+        us[v] = in[v] ? A.u[i + v] : 0.0f;
+        ca[v] = in[v] ? A.calcium[i + v] : 0.0;
+        const Grow32 G = grow32_of(A, in[v] && A.target ? A.target[i + v] : 0.0f);
+        flat[v] = G.flat;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            ds[t][v] = in[v] ? A.delta[t][i + v] : 0.0f;
+            xi[t][v] = -G.xi[t];
+            iz[t][v] = G.iz[t];
+        }
+    }
+    F2 x = f2(xs[0], xs[1]), u = f2(us[0], us[1]);
+    F2 d[3], mxi[3], izp[3], nup[3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        d[t] = f2(ds[t][0], ds[t][1]);
+        mxi[t] = f2_keep(xi[t][0], xi[t][1]);
+        izp[t] = f2_keep(iz[t][0], iz[t][1]);
+        nup[t] = f2_keep(nu[t], nu[t]);
+    }
+    const F2 sk1 = f2_keep(A.sk1, A.sk1), sk2 = f2_keep(A.sk2, A.sk2), ms = f2_keep(-A.s, -A.s), msa = f2_keep(-A.sa, -A.sa), mb = f2_keep(-A.b, -A.b);
+    const F2 two = f2_keep(2.0f, 2.0f), mone = f2_keep(-1.0f, -1.0f);
+    float in2[2] = { 0.0f, 0.0f };
+    for (uint32_t k = 0; k < nsteps; ++k) {
+        const u32x4 blk = noise_block_rk(rk0, rk1, step0 + k, local);
+        in2[0] = fmaf(0.0f, A.conductance, fmaf(A.noise_stddev, normal_from_bits24(blk.x >> 8), A.noise_mean));
+        in2[1] = fmaf(0.0f, A.conductance, fmaf(A.noise_stddev, normal_from_bits24(blk.z >> 8), A.noise_mean));
+        const F2 sc = f2(fmaf(A.s, in2[0], A.sk3), fmaf(A.s, in2[1], A.sk3));
+        bool done[2] = { false, false };
+        float uf[2] = { 0.0f, 0.0f };
+#pragma unroll
+        for (int it = 0; it < H; ++it) {
+            const F2 inc = f2_fma(x, f2_fma(sk1, x, sk2), f2_fma(ms, u, sc));
+            u = f2_fma(msa, f2_fma(mb, x, u), u);  // u + sa (b x - u), both signs turned
+            x = f2_add(x, inc);
+            float xa, xb;
+            f2_get(x, xa, xb);
+            if (__any_sync(0xFFFFFFFFu, fmaxf(xa, xb) >= A.v_spike)) {
+                float ua, ub;
+                f2_get(u, ua, ub);
+                if (xa >= A.v_spike) {
+                    uf[0] = done[0] ? uf[0] : ua + A.d;
+                    done[0] = true;
+                    xa = A.c;  // the neuron's later substeps are not used
+                }
+                if (xb >= A.v_spike) {
+                    uf[1] = done[1] ? uf[1] : ub + A.d;
+                    done[1] = true;
+                    xb = A.c;
+                }
+                x = f2(xa, xb);
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, done[0] || done[1])) {
+            float xa, xb, ua, ub;
+            f2_get(x, xa, xb);
+            f2_get(u, ua, ub);
+            x = f2(done[0] ? A.c : xa, done[1] ? A.c : xb);
+            u = f2(done[0] ? uf[0] : ua, done[1] ? uf[1] : ub);
+        }
+        float caf[2];
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            f_before[v] = f[v];
+            f[v] = en[v] ? done[v] : f[v];
+            ca[v] = fma(ca[v], A.ca_mul, done[v] ? A.ca_add : 0.0);
+            caf[v] = (float)ca[v];
+        }
+        const F2 cap = f2(caf[0], caf[1]);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const F2 q = f2_mul(f2_add(cap, mxi[t]), izp[t]);
+            float qa, qb;
+            f2_get(f2_mul(q, q), qa, qb);
+            F2 dz = f2_fma(two, f2(ex2_approx(-qa), ex2_approx(-qb)), mone);
+            if (((flat[0] | flat[1]) >> t) & 1u) {
+                float za, zb;
+                f2_get(dz, za, zb);
+                za = (flat[0] >> t) & 1u ? (caf[0] == A.eta[t] ? 0.0f : -1.0f) : za;
+                zb = (flat[1] >> t) & 1u ? (caf[1] == A.eta[t] ? 0.0f : -1.0f) : zb;
+                dz = f2(za, zb);
+            }
+            d[t] = f2_fma(dz, nup[t], d[t]);
+        }
+    }
+    f2_get(x, xs[0], xs[1]);
+    f2_get(u, us[0], us[1]);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        f2_get(d[t], ds[t][0], ds[t][1]);
+    }
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        if (!in[v]) {
+            continue;
+        }
+        if (en[v]) {
+            A.x[i + v] = xs[v];
+            A.u[i + v] = us[v];
+            A.calcium[i + v] = ca[v];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                A.delta[t][i + v] = ds[t][v];
+            }
+        }
+        if (A.input) {
+            A.input[i + v] = en[v] ? in2[v] : 0.0f;
+        }
+        A.fired_cur[i + v] = f[v] ? 1 : 0;
+        fired_before_last[i + v] = f_before[v] ? 1 : 0;
+    }
+}
+
+// k_activity_f32_steps with a neuron pair per thread (the Izhikevich model
+// with its substeps fixed at compile time, one network).  319 warp instructions
+// per step of 64 neurons against 374; 4M neurons: 24.8 -> 22.9 us per step, the
+// FMA pipe's heavy half (Philox's multiplies, half of the packed operations)
+// 74 % busy.
+template <int H, int BLOCK>
+__global__ void __launch_bounds__(BLOCK) k_activity_f32_pairs(Act32 A, const ActDesc* __restrict__ D, uint32_t nsteps,
+                                                              uint8_t* __restrict__ fired_before_last) {
+    pdl_wait_then_release();  // every input is the previous launch's output
+    const uint32_t i = 2u * (blockIdx.x * BLOCK + threadIdx.x);
+    const bool in[2] = { i < A.n, i + 1u < A.n };
+    pair_steps_f32<H>(A, D->base_step, nsteps, fired_before_last, i, in, i, A.nu1, A.rk0, A.rk1);
+}
+
 // Calcium and the growth deltas of the last m steps of one launch per step
 // from the spike history (row j: the chunk's step j), with the state in
 // registers: the same function and order as step by step, so the same bits.
@@ -1590,6 +1777,16 @@ void launch_act32_h(Ctx& c, const ActVariant& v, const Act32& A, uint32_t kstep)
 
 template <int H, int MODEL = RL_MODEL_IZHIKEVICH>
 void launch_steps32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_before_last) {
+    if constexpr (H > 0 && MODEL == RL_MODEL_IZHIKEVICH) {
+        // a batched context keeps a neuron per thread: in blocks of half its
+        // table's size the pairs are slower there (48 networks, 2.6M neurons:
+        // 13.6 us per step against 13.2)
+        if (!c.multi()) {
+            launch_pdl(&k_activity_f32_pairs<H, 128>, blocks_for((c.n + 1u) / 2u, 128), 128, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
+                       fired_before_last);
+            return;
+        }
+    }
     if (c.multi()) {
         launch_pdl(&k_activity_f32_steps<H, kNetBlock, true, MODEL>, c.num_net_blocks, kNetBlock, c.stream, A, (const ActDesc*)c.act_desc.p,
                    nsteps, fired_before_last);
