@@ -1283,6 +1283,26 @@ void run_activity_block(Ctx& c, uint32_t first_step, uint32_t nsteps) {
     if (nsteps == 0) {
         return;
     }
+    if (c.fused_work && c.step_fusion && c.graph.num_edges == 0 && (uint64_t)nsteps * c.n > c.fused_work && nsteps > 3) {
+        // the block in parts of equal length, each a launch of at least two steps
+        const uint64_t want = ((uint64_t)nsteps * c.n + c.fused_work - 1) / c.fused_work;
+        const uint32_t parts = (uint32_t)std::min<uint64_t>(want, nsteps / 2u);
+        const uint64_t limit = c.fused_work;
+        c.fused_work = 0;
+        uint32_t done = 0;
+        try {
+            for (uint32_t p = 0; p < parts; ++p) {
+                const uint32_t upto = (uint32_t)((uint64_t)nsteps * (p + 1u) / parts);
+                run_activity_block(c, first_step + done, upto - done);
+                done = upto;
+            }
+        } catch (...) {
+            c.fused_work = limit;
+            throw;
+        }
+        c.fused_work = limit;
+        return;
+    }
     c.act_block_len = nsteps;
     const bool edges = c.graph.num_edges > 0;
     if (edges) {

@@ -1247,6 +1247,12 @@ rl_status rl_set_graphs(void* ctx, int enable) {
     return rl::guarded(ctx, [&](Ctx& c) { c.use_graphs = enable != 0; });
 }
 
+// Serving (serve.cpp): fused blocks of steps in launches of at most `work`
+// neuron-steps.
+rl_status rl_internal_set_fused_work(void* ctx, uint64_t work) {
+    return rl::guarded(ctx, [&](Ctx& c) { c.fused_work = work; });
+}
+
 rl_status rl_set_step_fusion(void* ctx, int enable) {
     return rl::guarded(ctx, [&](Ctx& c) { c.step_fusion = enable != 0; });
 }

@@ -29,7 +29,14 @@
 
 #include "../../include/relearn_b200.h"
 
+extern "C" rl_status rl_internal_set_fused_work(void* ctx, uint64_t work);  // capi.cu
+
 namespace rl_serve {
+
+// Neuron-steps of a fused launch: 16 steps of a million neurons, about 0.1 ms
+// in the FP32 form, so that requests beside it wait no longer than that for an
+// SM; shorter launches would load and store the state too often.
+constexpr uint64_t kServeFusedWork = 16'000'000;
 
 using Clock = std::chrono::steady_clock;
 
@@ -236,11 +243,13 @@ struct Server {
         if ((st = rl_set_graphs(ctx, sc.use_graphs)) != RL_OK) {
             return fail(st, "rl_set_graphs");
         }
-        // One launch per activity step: a fused block of steps keeps its SMs
-        // for the whole block (about a millisecond for a large network), which
-        // holds back the kernels of the requests running beside it.
-        if ((st = rl_set_step_fusion(ctx, 0)) != RL_OK) {
-            return fail(st, "rl_set_step_fusion");
+        // Blocks of steps of a network without synapses in launches of at most
+        // kServeFusedWork neuron-steps: a whole block in one launch keeps its
+        // SMs for up to a millisecond and holds back the kernels of the
+        // requests running beside it, one launch per step takes up to three
+        // times as long.
+        if ((st = rl_internal_set_fused_work(ctx, kServeFusedWork)) != RL_OK) {
+            return fail(st, "rl_internal_set_fused_work");
         }
         if ((st = rl_autotune(ctx, sc.autotune)) != RL_OK) {
             return fail(st, "rl_autotune");
