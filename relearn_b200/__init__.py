@@ -592,8 +592,9 @@ class Network:
         self._check(self.lib.rl_set_graphs(self.h, int(on)))
 
     def set_step_fusion(self, on: bool = True):
-        """Blocks of activity steps of a network without synapses in one
-        launch (the default), or one launch per step; the same bits."""
+        """Blocks of activity steps of a network without synapses, or of one
+        with synapses whose neurons all have a resident thread, in one launch
+        (the default), or one launch per step; the same bits."""
         self._check(self.lib.rl_set_step_fusion(self.h, int(on)))
 
     def set_profiling(self, on: bool = True):

@@ -1,0 +1,155 @@
+// A block of activity steps of a network WITH synapses in one launch: the
+// parts shared by the FP64 (activity.cu) and FP32 (fp32.cu) kernels.
+//
+// A step's input needs every spike of the step before, so the thread blocks
+// meet at a barrier between steps.  One launch per step pays that as a launch
+// (launch, constant loads, state loads and drain, also when the network fills a
+// fraction of the device); here all thread blocks are resident together, the
+// state stays in registers, and the barrier is split: a block arrives when its
+// spikes are pushed and then does what does not depend on the others
+// (calcium, growth, the draws of the coming steps) before it waits.  Bound by
+// the chain of a step: pushed sum past L1, ten dependent substeps, the spikes'
+// edges, the barrier.  Microseconds per step, one launch per step -> here:
+// FP64 2,000 neurons 6.6 -> 3.3, 51,842 8.3 -> 3.8, 113,000 9.3 -> 4.9; FP32
+// 5.0 -> 2.5, 6.3 -> 3.3, 6.6 -> 3.6; AEIF FP64 100,003 12.0 -> 7.4.
+//
+// Up to kCoupledCluster thread blocks form one cluster and use the hardware's
+// cluster barrier (6,100 neurons: 3.4 us per step FP64, 2.6 FP32); more are
+// launched cooperatively (the launch fails rather than leave one of them out)
+// and count arrivals in device memory (6,200 neurons: 3.7 and 3.1 us).
+#pragma once
+
+#include "rl_context.cuh"
+
+namespace rl {
+
+constexpr int kCoupledBlock = 384;          // threads (neurons) per block, two blocks per SM
+constexpr unsigned kCoupledCluster = 16;    // blocks per cluster (8 are portable)
+constexpr uint32_t kCoupledPolls = 1u << 22;  // polls of a barrier before it gives up: some seconds
+
+#if defined(__CUDACC__)
+// This block's pushes of the step are issued by all its threads.
+template <bool CLUSTER>
+__device__ __forceinline__ void step_arrive(uint32_t* count) {
+    if constexpr (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    } else {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            // a release at device scope, which covers what the block's other
+            // threads wrote before the barrier above
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        }
+    }
+}
+
+// Waits until `arrivals` arrivals are counted; false (in every thread of the
+// block) if the bounded wait ran out, which is recorded in *err.
+template <bool CLUSTER>
+__device__ __forceinline__ bool step_wait(const uint32_t* count, uint32_t arrivals, uint32_t* err) {
+    if constexpr (CLUSTER) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    } else {
+        int late = 0;
+        if (threadIdx.x == 0) {
+            uint32_t polls = 0, seen = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+            } while ((int32_t)(seen - arrivals) < 0 && ++polls < kCoupledPolls);
+            if ((int32_t)(seen - arrivals) < 0) {
+                atomicOr(err, (uint32_t)DERR_TIMEOUT);
+                late = 1;
+            }
+        }
+        return __syncthreads_or(late) == 0;
+    }
+}
+
+// Neuron i's sum pushed at the step before, read past L1 (other SMs' atomics
+// wrote it) and cleared.
+template <typename T>
+__device__ __forceinline__ T take_pushed(T* in, uint32_t i) {
+    const T s = __ldcg(in + i);
+    if (s != 0) {
+        __stcg(in + i, (T)0);
+    }
+    return s;
+}
+
+__device__ __forceinline__ void add_weight(long long* p, int32_t w) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)(long long)w);  // two's complement: the signed sum
+}
+__device__ __forceinline__ void add_weight(int32_t* p, int32_t w) {
+    atomicAdd(p, w);
+}
+
+// The warp's spikes: each firing lane's out-edges o0 .. o1 go to their
+// targets' sums of the next step, four spikes at a time with eight lanes each,
+// so that the edges' dependent loads lie side by side.
+template <typename T>
+__device__ __forceinline__ void push_warp(bool f, uint32_t o0, uint32_t o1, const uint32_t* __restrict__ out_perm, const uint32_t* __restrict__ tgt,
+                                          const int32_t* __restrict__ w, T* next) {
+    uint32_t m = __ballot_sync(0xFFFFFFFFu, f);
+    const uint32_t g = (threadIdx.x & 31u) >> 3, sub = threadIdx.x & 7u;
+    while (m) {
+        const uint32_t m1 = m & (m - 1u), m2 = m1 & (m1 - 1u), m3 = m2 & (m2 - 1u);
+        const uint32_t mine = g == 0u ? m : (g == 1u ? m1 : (g == 2u ? m2 : m3));  // its lowest lane is the group's spike
+        const int s = mine ? __ffs((int)mine) - 1 : 0;
+        const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, o0, s), b1 = __shfl_sync(0xFFFFFFFFu, o1, s);
+        if (mine) {
+            for (uint32_t j = b0 + sub; j < b1; j += 8u) {
+                const uint32_t e = out_perm[j];
+                add_weight(next + tgt[e], w[e]);
+            }
+        }
+        m = m3 & (m3 - 1u);
+    }
+    __syncwarp();
+}
+#endif
+
+// Launches the coupled kernel of `steps` steps (its cluster form for few blocks) if all its
+// thread blocks can be resident together; false if not.
+template <typename... KArgs, typename... Args>
+bool launch_coupled(Ctx& c, uint32_t steps, void (*cluster_kernel)(KArgs...), void (*grid_kernel)(KArgs...), Args... args) {
+    const unsigned blocks = blocks_for(c.n, kCoupledBlock);
+    const bool cluster = blocks <= kCoupledCluster;
+    void (*kernel)(KArgs...) = cluster ? cluster_kernel : grid_kernel;
+    if (cluster) {
+        RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    } else {
+        int per_sm = 0;
+        RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, kCoupledBlock, 0));
+        if (blocks > (unsigned)per_sm * (unsigned)c.num_sms) {
+            return false;
+        }
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kCoupledBlock);
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = blocks;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PhaseScope ps(c, PH_ACTIVITY_KERNEL, steps);
+    if (cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...) != cudaSuccess) {
+        (void)cudaGetLastError();  // such a launch is not available here: the caller takes one launch per step
+        return false;
+    }
+    if (g_bind.launches) {
+        ++*g_bind.launches;
+    }
+    return true;
+}
+
+}  // namespace rl

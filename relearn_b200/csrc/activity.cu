@@ -21,6 +21,7 @@
 
 #include <cooperative_groups.h>
 
+#include "act_coupled.cuh"
 #include "rl_context.cuh"
 #include "rl_math.cuh"
 
@@ -621,16 +622,66 @@ __global__ void __launch_bounds__(256) k_calcium_growth(ActArgs A, uint32_t row0
 // Background draws a block-of-steps launch prepares per barrier round.
 constexpr int kDrawChunk = 10;
 
+// The standard normal draws of the m steps from stepc on (m <= kDrawChunk),
+// step stepc + k of this thread's neuron at s_z[k * BLOCK + threadIdx.x].  All
+// threads of the block call it; `parity` selects the shared tail-queue counter.
+// Lanes 2j and 2j + 1 hold a neuron pair (or its even member and an idle
+// lane), whose draws of a step come from one Philox block: the even lane
+// computes step k's block, the odd lane step k + 1's, and each hands the other
+// the two words it needs (the same words as a block per lane).
+template <int BLOCK, bool MULTI>
+__device__ __forceinline__ void draw_chunk64(bool on, uint32_t m, uint32_t stepc, uint64_t seed, uint32_t local, const uint32_t (&rk0)[10],
+                                             const uint32_t (&rk1)[10], uint32_t parity, double* s_z, uint16_t* s_who, uint32_t* s_cnt) {
+    constexpr int S = kDrawChunk;
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < S; k += 2) {
+        uint64_t b[2];
+        const uint32_t odd = lane & 1u;
+        // a batched context derives the round keys from the seed as it goes
+        // (twenty more registers would spill)
+        const u32x4 r = MULTI ? noise_block(seed, stepc + (uint32_t)k + odd, local) : noise_block_rk(rk0, rk1, stepc + (uint32_t)k + odd, local);
+        const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r.x : r.z, 1);
+        const uint32_t g1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r.y : r.w, 1);
+        const uint64_t got = ((uint64_t)g0 << 21) | (uint64_t)(g1 >> 11);
+        b[0] = odd ? got : (((uint64_t)r.x << 21) | (uint64_t)(r.y >> 11));
+        b[1] = odd ? (((uint64_t)r.z << 21) | (uint64_t)(r.w >> 11)) : got;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool use = on && (uint32_t)(k + h) < m;
+            const double p = uniform_from_bits53(b[h]);  // open (0, 1)
+            const bool tail = use && normal_in_tail(p);
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, tail);
+            uint32_t first = 0;
+            if (lane == 0 && mask) {
+                first = atomicAdd(&s_cnt[parity], (uint32_t)__popc(mask));
+            }
+            first = __shfl_sync(0xFFFFFFFFu, first, 0);
+            const uint32_t slot = (uint32_t)(k + h) * BLOCK + threadIdx.x;
+            if (tail) {
+                s_who[first + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = (uint16_t)slot;
+            }
+            s_z[slot] = tail ? p : (use ? normal_quantile_central(p) : 0.0);
+        }
+    }
+    __syncthreads();
+    const uint32_t cnt = s_cnt[parity];
+    for (uint32_t q = threadIdx.x; q < cnt; q += BLOCK) {
+        const uint32_t slot = s_who[q];
+        s_z[slot] = normal_quantile_tail(s_z[slot]);
+    }
+    if (threadIdx.x == 0) {
+        s_cnt[parity ^ 1u] = 0u;  // the next chunk's counter; nobody reads it before the barrier below
+    }
+    __syncthreads();
+}
+
 // One neuron's block of `nsteps` steps on registers (k_activity_steps): neuron
 // i of the context, `local` its index in its network, whose seed is `seed`
 // (its round keys rk0 / rk1 in a context with one network) and whose growth
 // rates are nu.  A lane with `in` false holds no
-// neuron but still draws for its lane pair.  Lanes 2j and 2j + 1 hold a neuron
-// pair (or its even member and an idle lane), whose draws of a step come from
-// one Philox block: the even lane computes step k's block, the odd lane step
-// k + 1's, and each hands the other the two words it needs (the same words as
-// a block per lane).  `parity` selects the shared tail-queue counter of the
-// next chunk.
+// neuron but still draws for its lane pair.  `parity` selects the shared
+// tail-queue counter of the next chunk.
 template <int BLOCK, int H, int MODEL, bool MULTI, bool TOP>
 __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* __restrict__ D, uint32_t nsteps,
                                                uint8_t* __restrict__ fired_before_last, uint32_t i, bool in, uint64_t seed, uint32_t local,
@@ -638,7 +689,6 @@ __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* 
                                                uint16_t* s_who, uint32_t* s_cnt) {
     constexpr int S = kDrawChunk;
     const uint32_t step0 = D->base_step;
-    const uint32_t lane = threadIdx.x & 31u;
     const bool on = in && A.enabled[i];
     double xv = 0.0, uv = 0.0, ca = 0.0, tgt = 0.0, d0 = 0.0, d1 = 0.0, d2 = 0.0, input = 0.0;
     uint8_t f = 0;
@@ -658,46 +708,7 @@ __device__ __forceinline__ void neuron_steps64(const ActArgs& A, const ActDesc* 
     for (uint32_t k0 = 0; k0 < nsteps; k0 += S, parity ^= 1u) {
         const uint32_t m = nsteps - k0 < (uint32_t)S ? nsteps - k0 : (uint32_t)S;
         const uint32_t stepc = step0 + k0;
-#pragma unroll
-        for (int k = 0; k < S; k += 2) {
-            uint64_t b[2];
-            const uint32_t odd = lane & 1u;
-            // a batched context derives the round keys from the seed as it goes
-            // (twenty more registers would spill)
-            const u32x4 r = MULTI ? noise_block(seed, stepc + (uint32_t)k + odd, local) : noise_block_rk(rk0, rk1, stepc + (uint32_t)k + odd, local);
-            const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r.x : r.z, 1);
-            const uint32_t g1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r.y : r.w, 1);
-            const uint64_t got = ((uint64_t)g0 << 21) | (uint64_t)(g1 >> 11);
-            b[0] = odd ? got : (((uint64_t)r.x << 21) | (uint64_t)(r.y >> 11));
-            b[1] = odd ? (((uint64_t)r.z << 21) | (uint64_t)(r.w >> 11)) : got;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const bool use = on && (uint32_t)(k + h) < m;
-                const double p = uniform_from_bits53(b[h]);  // open (0, 1)
-                const bool tail = use && normal_in_tail(p);
-                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, tail);
-                uint32_t first = 0;
-                if (lane == 0 && mask) {
-                    first = atomicAdd(&s_cnt[parity], (uint32_t)__popc(mask));
-                }
-                first = __shfl_sync(0xFFFFFFFFu, first, 0);
-                const uint32_t slot = (uint32_t)(k + h) * BLOCK + threadIdx.x;
-                if (tail) {
-                    s_who[first + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = (uint16_t)slot;
-                }
-                s_z[slot] = tail ? p : (use ? normal_quantile_central(p) : 0.0);
-            }
-        }
-        __syncthreads();
-        const uint32_t cnt = s_cnt[parity];
-        for (uint32_t q = threadIdx.x; q < cnt; q += BLOCK) {
-            const uint32_t slot = s_who[q];
-            s_z[slot] = normal_quantile_tail(s_z[slot]);
-        }
-        if (threadIdx.x == 0) {
-            s_cnt[parity ^ 1u] = 0u;  // the next chunk's counter; nobody reads it before the barrier below
-        }
-        __syncthreads();
+draw_chunk64<BLOCK, MULTI>(on, m, stepc, seed, local, rk0, rk1, parity, s_z, s_who, s_cnt);
         bool piped = false;
         if constexpr (MODEL == RL_MODEL_IZHIKEVICH && H > 0) {
             if (on && A.uniform_target) {
@@ -788,6 +799,118 @@ __global__ void __launch_bounds__(BLOCK, (MULTI ? 640 : 768) / BLOCK) k_activity
             neuron_steps64<BLOCK, H, MODEL, false, TOP>(A, D, nsteps, fired_before_last, i, i < A.n, A.seed1, i, nu, A.rk0, A.rk1, parity, s_z,
                                                    s_who, s_cnt);
         }
+    }
+}
+
+// A block of `nsteps` steps of a network with synapses in one launch
+// (act_coupled.cuh): one neuron per thread, every thread block resident.  The
+// operations are k_activity's and k_calcium_growth's in their order, so the
+// bits are theirs.  Bound by the chain of one step (read the pushed sum past
+// L1, ten dependent substeps, push, barrier), not by a pipe.
+template <int BLOCK, int H, int MODEL, bool TOP, bool CLUSTER>
+__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled(ActArgs A, const ActDesc* __restrict__ D, uint32_t nsteps,
+                                                                         uint8_t* __restrict__ fired_before_last, uint32_t* bar, uint32_t* err) {
+    __shared__ double s_z[kDrawChunk * BLOCK];
+    __shared__ uint16_t s_who[kDrawChunk * BLOCK];
+    __shared__ uint32_t s_cnt[2];
+    if (threadIdx.x < 2) {
+        s_cnt[threadIdx.x] = 0u;
+    }
+    const uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
+    const bool in = i < A.n;
+    const bool on = in && A.enabled[i];
+    const uint32_t step0 = D->base_step;
+    const uint32_t* __restrict__ out_perm = D->out_perm;
+    const uint32_t* __restrict__ tgt_of = D->tgt;
+    const int32_t* __restrict__ w_of = D->w;
+    const Nu nu{ { A.nu1[0], A.nu1[1], A.nu1[2] } };
+    double xv = 0.0, uv = 0.0, ca = 0.0, tgt = 0.0, d0 = 0.0, d1 = 0.0, d2 = 0.0, input = 0.0;
+    uint8_t f = 0;
+    uint32_t o0 = 0, o1 = 0;
+    if (in) {
+        f = A.fired_prev[i];
+        d0 = A.delta0[i];
+        d1 = A.delta1[i];
+        d2 = A.delta2[i];
+        o0 = D->out_off[i];
+        o1 = D->out_off[i + 1];
+    }
+    if (on) {
+        xv = A.x[i];
+        uv = A.u[i];
+        ca = A.calcium[i];
+        tgt = A.uniform_target ? 0.0 : A.target[i];
+    }
+    uint8_t f_before = f;
+    __syncthreads();
+    uint32_t parity = 0;
+    for (uint32_t k0 = 0; k0 < nsteps; k0 += kDrawChunk, parity ^= 1u) {
+        const uint32_t m = nsteps - k0 < (uint32_t)kDrawChunk ? nsteps - k0 : (uint32_t)kDrawChunk;
+        draw_chunk64<BLOCK, false>(on, m, step0 + k0, A.seed1, i, A.rk0, A.rk1, parity, s_z, s_who, s_cnt);
+        for (uint32_t j = 0; j < m; ++j) {
+            const uint32_t k = k0 + j, step = step0 + k;
+            long long isum = 0;
+            if (k == 0) {
+                isum = on ? synaptic_sum(A, D, i) : 0;
+            } else {
+                if (!step_wait<CLUSTER>(bar, k * gridDim.x, err)) {
+                    return;
+                }
+                if (in) {
+                    isum = take_pushed(A.syn_in[step & 1u], i);
+                }
+            }
+            if (on) {
+                input = step_input(A, isum, s_z[j * BLOCK + threadIdx.x]);
+                f_before = f;
+                if constexpr (MODEL == RL_MODEL_IZHIKEVICH && H > 0) {
+                    f = izhikevich_frozen<H, TOP>(A, input, xv, uv);
+                } else {
+                    f = model_step<H, MODEL>(A, step, A.seed1, i, input, xv, uv);
+                }
+            }
+            __syncwarp();
+            if (k + 1 < nsteps) {
+                // a disabled neuron keeps its flag, and its targets read it
+                push_warp(f != 0, o0, o1, out_perm, tgt_of, w_of, A.syn_in[(step + 1u) & 1u]);
+                step_arrive<CLUSTER>(bar);
+            }
+            if (on) {
+                bool flat = false;
+                if constexpr (H > 0) {
+                    if (A.uniform_target) {
+                        calcium_growth_flat<H, false>(A, f, nu, ca, d0, d1, d2);
+                        flat = true;
+                    }
+                }
+                if (!flat) {
+                    ca = calcium_step<H>(A, f, ca);
+                    d0 = d0 + growth_step(A, 0, ca, tgt, nu);
+                    d1 = d1 + growth_step(A, 1, ca, tgt, nu);
+                    d2 = d2 + growth_step(A, 2, ca, tgt, nu);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    if (on) {
+        A.x[i] = xv;
+        A.u[i] = uv;
+        A.calcium[i] = ca;
+        A.delta0[i] = d0;
+        A.delta1[i] = d1;
+        A.delta2[i] = d2;
+    } else if (in) {
+        A.delta0[i] = d0 + 0.0;
+        A.delta1[i] = d1 + 0.0;
+        A.delta2[i] = d2 + 0.0;
+    }
+    if (in) {
+        if (A.input) {
+            A.input[i] = on ? input : 0.0;
+        }
+        A.fired_cur[i] = f;
+        fired_before_last[i] = f_before;
     }
 }
 
@@ -1093,6 +1216,37 @@ void launch_calcium_growth64(Ctx& c, uint32_t row0, uint32_t m, cudaStream_t st)
     RL_LAUNCH_CHECK();
 }
 
+template <int H, int MODEL, bool TOP = false>
+bool launch_coupled64_m(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_before_last) {
+    return launch_coupled(c, nsteps, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, true>, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, false>, A,
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p);
+}
+
+template <int H>
+bool launch_coupled64(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_before_last) {
+    switch (c.cfg.neuron_model) {
+        case RL_MODEL_POISSON:
+            return launch_coupled64_m<H, RL_MODEL_POISSON>(c, A, nsteps, fired_before_last);
+        case RL_MODEL_FITZHUGH_NAGUMO:
+            return launch_coupled64_m<H, RL_MODEL_FITZHUGH_NAGUMO>(c, A, nsteps, fired_before_last);
+        case RL_MODEL_AEIF:
+            return launch_coupled64_m<H, RL_MODEL_AEIF>(c, A, nsteps, fired_before_last);
+        default:
+            return H > 0 && A.spike_hi != 0u ? launch_coupled64_m<H, RL_MODEL_IZHIKEVICH, true>(c, A, nsteps, fired_before_last)
+                                             : launch_coupled64_m<H, RL_MODEL_IZHIKEVICH>(c, A, nsteps, fired_before_last);
+    }
+}
+
+// The whole block of nsteps steps in one launch, a network with synapses;
+// false if its thread blocks cannot all be resident.
+bool launch_activity_fp64_coupled(Ctx& c, uint32_t nsteps) {
+    const int p0 = c.nr.cur & 1;
+    const ActArgs A = act64_args(c, nsteps - 1, c.nr.fired[p0].p, c.nr.fired[(p0 + (int)nsteps) & 1].p);
+    uint8_t* before_last = c.nr.fired[(p0 + (int)nsteps - 1) & 1].p;
+    return c.cfg.h_model == 10 && c.cfg.h_calcium == 10 ? launch_coupled64<10>(c, A, nsteps, before_last)
+                                                        : launch_coupled64<0>(c, A, nsteps, before_last);
+}
+
 // The whole block of nsteps steps in one launch (a network without synapses).
 void launch_activity_fp64_steps(Ctx& c, uint32_t nsteps) {
     const int p0 = c.nr.cur & 1;
@@ -1107,8 +1261,9 @@ void launch_activity_fp64_steps(Ctx& c, uint32_t nsteps) {
 
 namespace {
 
-__global__ void k_set_desc(ActDesc* D, ActDesc v) {
+__global__ void k_set_desc(ActDesc* D, ActDesc v, uint32_t* bar) {
     *D = v;
+    *bar = 0u;  // the arrivals of a coupled launch
 }
 
 void launch_step(Ctx& c, uint32_t kstep, const ActVariant& v) {
@@ -1279,6 +1434,28 @@ void drop_activity_graphs(Ctx& c) {
     }
 }
 
+namespace {
+
+void finish_block(Ctx& c, uint32_t nsteps) {
+    c.nr.cur ^= (int)(nsteps & 1u);
+    c.stats.activity_steps += nsteps;
+    if (c.copy_stream) {
+        issue_snapshots(c);  // the block is queued: snapshot copies now overlap it
+    }
+}
+
+// A block of steps of a network with synapses in one launch (act_coupled.cuh)
+// where every neuron has a resident thread; false if it is to run one launch
+// per step.  In a serving context only within the work of one fused launch.
+bool run_coupled_block(Ctx& c, uint32_t nsteps) {
+    if (!c.step_fusion || nsteps < 2 || c.multi() || (c.fused_work && (uint64_t)nsteps * c.n > c.fused_work)) {
+        return false;
+    }
+    return is_fp32(c) ? launch_activity_f32_coupled(c, nsteps) : launch_activity_fp64_coupled(c, nsteps);
+}
+
+}  // namespace
+
 void run_activity_block(Ctx& c, uint32_t first_step, uint32_t nsteps) {
     if (nsteps == 0) {
         return;
@@ -1310,9 +1487,14 @@ void run_activity_block(Ctx& c, uint32_t first_step, uint32_t nsteps) {
     }
     const ActDesc v{ first_step, edges ? 1u : 0u, c.graph.offsets.p, c.graph.src.p, c.graph.weight.p, nsteps, c.graph.out_off.p, c.graph.out_perm.p,
                      c.graph.tgt.p };
-    k_set_desc<<<1, 1, 0, c.stream>>>(c.act_desc.p, v);
+    k_set_desc<<<1, 1, 0, c.stream>>>(c.act_desc.p, v, c.act_bar.p);
     RL_LAUNCH_CHECK();
     const bool fused = c.step_fusion && c.graph.num_edges == 0 && nsteps > 1;
+    // (a requested tuning still times the shapes of one launch per step first)
+    if (edges && c.tune.act_state != TUNE_REQUESTED && run_coupled_block(c, nsteps)) {
+        finish_block(c, nsteps);
+        return;
+    }
     if (!fused) {
         ensure_spike_hist(c);
         if (nsteps > kGrowthChunk && c.growth_stream == nullptr) {
@@ -1331,6 +1513,10 @@ void run_activity_block(Ctx& c, uint32_t first_step, uint32_t nsteps) {
         }
         c.tune.act_state = TUNE_DONE;
         drop_activity_graphs(c);
+        if (edges && run_coupled_block(c, nsteps)) {
+            finish_block(c, nsteps);
+            return;
+        }
     }
     const bool graph = !fused && c.use_graphs && c.stream != nullptr && nsteps > 1 && nsteps == c.cfg.plasticity_interval;
     // One launch per step; calcium and growth of each chunk of kGrowthChunk
@@ -1419,11 +1605,7 @@ void run_activity_block(Ctx& c, uint32_t first_step, uint32_t nsteps) {
             step_and_growth(k);
         }
     }
-    c.nr.cur ^= (int)(nsteps & 1u);
-    c.stats.activity_steps += nsteps;
-    if (c.copy_stream) {
-        issue_snapshots(c);  // the block is queued: snapshot copies now overlap it
-    }
+    finish_block(c, nsteps);
 }
 
 namespace {

@@ -357,6 +357,7 @@ void create(Ctx& c, const rl_config& k, const rl_network* nets = nullptr, uint32
     RL_CUDA_TRY(cudaMemsetAsync(c.graph.offsets.p, 0, (n + 1) * sizeof(uint32_t), c.stream));
     c.to_delete.alloc(n);
     c.act_desc.alloc(1);
+    c.act_bar.alloc(1);
     c.err.alloc(1);
     RL_CUDA_TRY(cudaMemsetAsync(c.err.p, 0, sizeof(uint32_t), c.stream));
     c.commit_cnt.alloc(4);

@@ -24,6 +24,7 @@
 // formed synapses.
 #include "bh_bins.cuh"
 #include "bh_eval.cuh"
+#include "act_coupled.cuh"
 #include "rl_context.cuh"
 #include "rl_math.cuh"
 
@@ -601,6 +602,97 @@ __global__ void __launch_bounds__(BLOCK) k_activity_f32_steps(Act32 A, const Act
             const uint32_t i = base + threadIdx.x;
             neuron_steps_f32<H, false, MODEL>(A, D, nsteps, fired_before_last, i, i < A.n, i, true, A.nu1, A.rk0, A.rk1);
         }
+    }
+}
+
+// A block of `nsteps` steps of a network with synapses in one launch
+// (act_coupled.cuh): one neuron per thread, every thread block resident.  The
+// operations are k_activity_f32's and k_calcium_growth_f32's in their order,
+// so the bits are theirs.
+template <int BLOCK, int H, int MODEL, bool CLUSTER>
+__global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled(Act32 A, const ActDesc* __restrict__ D, uint32_t nsteps,
+                                                                             uint8_t* __restrict__ fired_before_last, uint32_t* bar, uint32_t* err) {
+    const uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
+    const bool in = i < A.n;
+    const bool en = in && A.enabled[i] != 0;
+    const uint32_t step0 = D->base_step;
+    const uint32_t* __restrict__ out_perm = D->out_perm;
+    const uint32_t* __restrict__ tgt_of = D->tgt;
+    const int32_t* __restrict__ w_of = D->w;
+    uint8_t f = 0;
+    float x = 0.0f, u = 0.0f, tg = 0.0f, input = 0.0f;
+    double ca = 0.0;
+    float d[3] = { 0.0f, 0.0f, 0.0f };
+    uint32_t o0 = 0, o1 = 0;
+    if (in) {
+        if (A.target) {
+            tg = A.target[i];
+        }
+        f = A.fired_prev[i];
+        x = A.x[i];
+        u = A.u[i];
+        ca = A.calcium[i];
+        d[0] = A.delta[0][i];
+        d[1] = A.delta[1][i];
+        d[2] = A.delta[2][i];
+        o0 = D->out_off[i];
+        o1 = D->out_off[i + 1];
+    }
+    uint8_t f_before = f;
+    const Grow32 G = grow32_of(A, tg);
+    const uint32_t odd = threadIdx.x & 1u;
+    uint32_t word = 0, word_next = 0;
+    for (uint32_t k = 0; k < nsteps; ++k) {
+        const uint32_t step = step0 + k;
+        if ((k & 1u) == 0u) {
+            // two steps' draws: one Philox block per lane, as neuron_steps_f32 shares them
+            const u32x4 blk = noise_block_rk(A.rk0, A.rk1, step + odd, i);
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? blk.x : blk.z, 1);
+            const uint32_t own = odd ? blk.z : blk.x;
+            word = odd ? got : own;
+            word_next = odd ? own : got;
+        } else {
+            word = word_next;
+        }
+        uint32_t k24p = 0;
+        if (MODEL == RL_MODEL_POISSON) {
+            k24p = philox4x32_10_rk(u32x4{ step, i, 0u, (uint32_t)STREAM_POISSON << 24 }, A.rk0, A.rk1).x >> 8;
+        }
+        int pushed = 0;
+        if (k > 0) {
+            if (!step_wait<CLUSTER>(bar, k * gridDim.x, err)) {
+                return;
+            }
+            if (in) {
+                pushed = take_pushed(A.syn_in[step & 1u], i);
+            }
+        }
+        uint8_t fired;
+        neuron_f32<H, MODEL, true, false>(A, D, i, en, f, word >> 8, k24p, A.nu1, G, x, u, ca, d, input, fired, k == 0, pushed);
+        f_before = f;
+        f = fired;
+        __syncwarp();
+        if (k + 1 < nsteps) {
+            push_warp(f != 0, o0, o1, out_perm, tgt_of, w_of, A.syn_in[(step + 1u) & 1u]);
+            step_arrive<CLUSTER>(bar);
+        }
+        if (en) {
+            calcium_growth_f32(A, f, A.nu1, G, ca, d);
+        }
+        __syncwarp();
+    }
+    if (in) {
+        A.x[i] = x;
+        A.u[i] = u;
+        A.calcium[i] = ca;
+        A.delta[0][i] = d[0];
+        A.delta[1][i] = d[1];
+        A.delta[2][i] = d[2];
+        if (A.input) {
+            A.input[i] = input;
+        }
+        A.fired_cur[i] = f;
+        fired_before_last[i] = f_before;
     }
 }
 
@@ -1894,6 +1986,35 @@ void launch_activity_f32(Ctx& c, uint32_t kstep, const uint8_t* fired_prev, uint
         launch_act32_h<10>(c, v, A, kstep);
     } else {
         launch_act32_h<0>(c, v, A, kstep);
+    }
+}
+
+namespace {
+
+template <int H, int MODEL>
+bool launch_coupled32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_before_last) {
+    return launch_coupled(c, nsteps, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, true>, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, false>, A,
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p);
+}
+
+}  // namespace
+
+// The whole block of nsteps steps in one launch, a network with synapses;
+// false if its thread blocks cannot all be resident.
+bool launch_activity_f32_coupled(Ctx& c, uint32_t nsteps) {
+    const int p0 = c.nr.cur & 1;
+    const Act32 A = act32_args(c, nsteps - 1, c.nr.fired[p0].p, c.nr.fired[(p0 + (int)nsteps) & 1].p);
+    uint8_t* before_last = c.nr.fired[(p0 + (int)nsteps - 1) & 1].p;
+    switch (c.cfg.neuron_model) {
+        case RL_MODEL_POISSON:
+            return launch_coupled32<0, RL_MODEL_POISSON>(c, A, nsteps, before_last);
+        case RL_MODEL_FITZHUGH_NAGUMO:
+            return launch_coupled32<0, RL_MODEL_FITZHUGH_NAGUMO>(c, A, nsteps, before_last);
+        case RL_MODEL_AEIF:
+            return launch_coupled32<0, RL_MODEL_AEIF>(c, A, nsteps, before_last);
+        default:
+            return c.cfg.h_model == 10 ? launch_coupled32<10, RL_MODEL_IZHIKEVICH>(c, A, nsteps, before_last)
+                                       : launch_coupled32<0, RL_MODEL_IZHIKEVICH>(c, A, nsteps, before_last);
     }
 }
 

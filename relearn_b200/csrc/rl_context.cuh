@@ -344,6 +344,7 @@ struct Ctx {
     cudaStream_t own_stream = nullptr;  // the context's own stream
     PhaseTimer timer;
     DBuf<ActDesc> act_desc;
+    DBuf<uint32_t> act_bar;  // arrivals at the barriers of a coupled launch (act_coupled.cuh)
     // synaptic sums pushed by the spikes of a step, by step parity (FP64 form:
     // syn_in64, FP32 form: syn_in32); zero at every block boundary
     DBuf<long long> syn_in64[2];
@@ -487,6 +488,8 @@ void launch_activity_fp64(Ctx& c, uint32_t k, const uint8_t* fired_prev, uint8_t
 // A block of nsteps steps in one launch; only for a network without synapses.
 void launch_activity_f32_steps(Ctx& c, uint32_t nsteps);
 void launch_activity_fp64_steps(Ctx& c, uint32_t nsteps);
+bool launch_activity_f32_coupled(Ctx& c, uint32_t nsteps);
+bool launch_activity_fp64_coupled(Ctx& c, uint32_t nsteps);
 uint64_t run_commit_f32(Ctx& c, int type);
 void pack_tree_f32(Ctx& c);
 void launch_search_f32(Ctx& c, int type, const uint32_t* seg_warp, const uint64_t* seg_begin, const uint64_t* seg_end, const uint32_t* seg_net,
