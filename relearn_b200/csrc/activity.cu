@@ -1784,9 +1784,10 @@ void launch_commit_guarded(Ctx& c, int type) {
     RL_LAUNCH_CHECK();
 }
 
-uint64_t run_commit(Ctx& c, int type) {
+void queue_commit(Ctx& c, int type, unsigned long long* bound) {
     if (is_fp32(c)) {
-        return run_commit_f32(c, type);
+        launch_commit_f32(c, type, bound, nullptr, 0);
+        return;
     }
     CommitArgs A;
     A.n = c.n;
@@ -1797,18 +1798,11 @@ uint64_t run_commit(Ctx& c, int type) {
     A.vacant = c.nr.vacant[type].p;
     A.retract = c.cfg.retract_ratio[type];
     A.to_delete = c.to_delete.p;
-    unsigned long long* d_del = reinterpret_cast<unsigned long long*>(c.counters.p) + 1;
-    RL_CUDA_TRY(cudaMemsetAsync(d_del, 0, sizeof(unsigned long long), c.stream));
-    A.total = d_del;
+    A.total = bound;
     A.guard = nullptr;
     A.guard_n = 0;
     k_commit<<<blocks_for(c.n, 256), 256, 0, c.stream>>>(A);
     RL_LAUNCH_CHECK();
-    unsigned long long h = 0;
-    RL_CUDA_TRY(cudaMemcpyAsync(&h, d_del, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
-    RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
-    c.stats.bound_to_delete += h;
-    return h;
 }
 
 }  // namespace rl

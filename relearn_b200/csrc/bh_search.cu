@@ -1013,7 +1013,7 @@ void launch_wide(Ctx& c, const SearchArgs (&a)[2], const uint32_t (&warps)[2]) {
             launch_bins_kernel<false>(c, A);
         }
     }
-    uint32_t left[4] = { 0, 0, 0, 0 };
+    uint32_t* left = c.read_slot() + kReadA;
     RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     RL_CUDA_TRY(cudaStreamSynchronize(st));
     const uint64_t open = (uint64_t)left[0] + left[1];
@@ -1156,12 +1156,11 @@ void run_search(Ctx& c, uint32_t step) {
     // one scan over both halves: excitatory offsets, then inhibitory offsets
     // counted on from the last excitatory search
     const uint32_t* dtot = exclusive_scan_u32_async(S.counts.p, S.counts.p, 2 * (uint64_t)n, c.prim, st);
-    uint32_t h[2] = { 0, 0 };
-    RL_CUDA_TRY(cudaMemcpyAsync(&h[0], cnt_inh, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    RL_CUDA_TRY(cudaMemcpyAsync(&h[1], dtot, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    RL_CUDA_TRY(cudaMemcpyAsync(c.read_slot() + kReadA, cnt_inh, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    RL_CUDA_TRY(cudaMemcpyAsync(c.read_slot() + kReadB, dtot, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     RL_CUDA_TRY(cudaStreamSynchronize(st));
-    const uint64_t num_exc = h[0];
-    const uint64_t m = h[1];
+    const uint64_t num_exc = c.read_slot()[kReadA];
+    const uint64_t m = c.read_slot()[kReadB];
     const uint64_t num_inh = m - num_exc;
     S.num_searches = m;
     S.num_exc = num_exc;
@@ -1329,18 +1328,24 @@ void run_search(Ctx& c, uint32_t step) {
     }
     k_req_count<<<blocks_for(n, 256), 256, 0, st>>>(n, S.first_fail.p, c.nr.search_vacant.p, c.nr.enabled.p, S.req_count.p);
     RL_LAUNCH_CHECK();
-    const uint64_t nreq = exclusive_scan_u32(S.req_count.p, S.req_off.p, n, c.prim, st);
-    S.num_requests = nreq;
-    S.req_tgt.ensure(nreq);
-    S.req_src.ensure(nreq);
-    S.req_j.ensure(nreq);
-    S.req_sig.ensure(nreq);
+    // the requests' number is read with the error word, behind their scatter:
+    // there is at most one per search
+    const uint32_t* dreq = exclusive_scan_u32_async(S.req_count.p, S.req_off.p, n, c.prim, st);
+    RL_CUDA_TRY(cudaMemcpyAsync(c.read_slot() + kReadA, dreq, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    S.req_tgt.ensure(m);
+    S.req_src.ensure(m);
+    S.req_j.ensure(m);
+    S.req_sig.ensure(m);
     if (m > 0) {
         k_req_scatter<<<blocks_for(m, 256), 256, 0, st>>>(m, S.src.p, S.jj.p, S.target.p, S.first_fail.p, S.req_off.p, c.nr.signal.p, S.req_tgt.p,
                                                           S.req_src.p, S.req_j.p, S.req_sig.p);
         RL_LAUNCH_CHECK();
     }
-    check_device_error(c, "barnes-hut search");
+    queue_error_read(c);
+    RL_CUDA_TRY(cudaStreamSynchronize(st));
+    const uint64_t nreq = c.read_slot()[kReadA];
+    S.num_requests = nreq;
+    raise_device_error(c, "barnes-hut search");
     c.stats.searches += m;
     c.stats.requests += nreq;
 }

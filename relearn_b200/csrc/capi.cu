@@ -60,10 +60,22 @@ static void resolve_timers(Ctx& c) {
     }
 }
 
+uint32_t* Ctx::read_slot() const {
+    return reinterpret_cast<uint32_t*>(h_commit + kReadSlot);
+}
+
 void check_device_error(Ctx& c, const char* phase) {
-    uint32_t h = 0;
-    RL_CUDA_TRY(cudaMemcpyAsync(&h, c.err.p, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
+    queue_error_read(c);
     RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    raise_device_error(c, phase);
+}
+
+void queue_error_read(Ctx& c) {
+    RL_CUDA_TRY(cudaMemcpyAsync(c.read_slot() + kReadError, c.err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+}
+
+void raise_device_error(Ctx& c, const char* phase) {
+    const uint32_t h = c.read_slot()[kReadError];
     if (h == 0) {
         return;
     }
@@ -261,7 +273,7 @@ std::vector<unsigned long long*> g_pinned_free;
 unsigned long long* pinned_slot_take() {
     std::lock_guard<std::mutex> lk(g_pinned_mu);
     if (g_pinned_free.empty()) {
-        constexpr size_t kSlot = 4, kSlots = 512;  // 16 KiB per page
+        constexpr size_t kSlot = kReadSlot + 4, kSlots = 512;  // 64 KiB per page
         unsigned long long* page = nullptr;
         RL_CUDA_TRY(cudaMallocHost(&page, kSlot * kSlots * sizeof(unsigned long long)));
         for (size_t k = 0; k < kSlots; ++k) {
@@ -360,8 +372,9 @@ void create(Ctx& c, const rl_config& k, const rl_network* nets = nullptr, uint32
     c.act_bar.alloc(1);
     c.err.alloc(1);
     RL_CUDA_TRY(cudaMemsetAsync(c.err.p, 0, sizeof(uint32_t), c.stream));
-    c.commit_cnt.alloc(4);
+    c.commit_cnt.alloc(kCommitCounts);
     c.h_commit = pinned_slot_take();
+    RL_CUDA_TRY(cudaEventCreateWithFlags(&c.commit_read, cudaEventDisableTiming));
     c.counters.alloc(4);
     RL_CUDA_TRY(cudaMemsetAsync(c.counters.p, 0, 4 * sizeof(uint64_t), c.stream));
     setup_nets(c, nets, num_nets);
@@ -389,7 +402,7 @@ void plasticity_update(Ctx& c, uint32_t step) {
         // sequential path has to take over.
         {
             PhaseScope ps(c, PH_COMMIT);
-            RL_CUDA_TRY(cudaMemsetAsync(c.commit_cnt.p, 0, 4 * sizeof(unsigned long long), c.stream));
+            RL_CUDA_TRY(cudaMemsetAsync(c.commit_cnt.p, 0, kCommitCounts * sizeof(unsigned long long), c.stream));
             if (!launch_commit_all(c)) {
                 for (int t = 0; t < 3; ++t) {
                     launch_commit_guarded(c, t);
@@ -419,18 +432,35 @@ void plasticity_update(Ctx& c, uint32_t step) {
         const int first = h[0] ? 0 : (h[1] ? 1 : (h[2] ? 2 : 3));
         // deletions change vacant axons: then the search counts them itself
         c.no_searches = first == 3 && h[3] == 0;
+        // The deletions and the later types' commits go out in order without
+        // a host read between them (a deletion pass over no bound elements
+        // ends at its first load), the octree update behind them; their
+        // counts and the error word are read once, while that update runs.
         if (first < 3) {
             PhaseScope ps(c, PH_COMMIT);
-            c.stats.synapses_deleted += run_deletion(c, step, first);
+            rebuild_graph(c);
+            unsigned long long* cnt = c.commit_cnt.p;
+            queue_deletion(c, step, first, cnt + 7 + first);
             for (int t = first + 1; t < 3; ++t) {
-                if (run_commit(c, t) > 0) {
-                    c.stats.synapses_deleted += run_deletion(c, step, t);
-                }
+                queue_commit(c, t, cnt + 4 + t);
+                queue_deletion(c, step, t, cnt + 7 + t);
             }
+            RL_CUDA_TRY(cudaMemcpyAsync(c.h_commit + 4, cnt + 4, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.stream));
+            queue_error_read(c);
+            RL_CUDA_TRY(cudaEventRecord(c.commit_read, c.stream));
         }
         if (first < 3 || !speculate) {
             PhaseScope ps(c, PH_TREE_UPDATE);
             update_tree(c);
+        }
+        if (first < 3) {
+            RL_CUDA_TRY(cudaEventSynchronize(c.commit_read));
+            raise_device_error(c, "synapse deletion");
+            for (int t = 0; t < 3; ++t) {
+                c.stats.bound_to_delete += h[4 + t];
+                c.stats.synapses_deleted += h[7 + t];
+                note_deleted(c, h[7 + t]);
+            }
         }
         c.deleted_last = first < 3;
     }
@@ -783,6 +813,10 @@ void discard(Ctx* c) {
         if (g) {
             cudaGraphExecDestroy(g);
         }
+    }
+    if (c->commit_read) {
+        cudaEventDestroy(c->commit_read);
+        c->commit_read = nullptr;
     }
     if (c->h_commit) {
         pinned_slot_give(c->h_commit);

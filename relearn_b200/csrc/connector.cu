@@ -467,15 +467,19 @@ uint64_t run_connector(Ctx& c, uint32_t step, bool bind_axons) {
     // compact accepted into the new-edge buffer (sorted-position order)
     DBuf<uint32_t>& pos = S.accept_pos;
     pos.fit(m);
-    const uint64_t created = exclusive_scan_u32(S.accepted.p, pos.p, m, c.prim, st);
-    const uint64_t need = G.num_new + created;
+    // their count is read with the error word, behind the compaction: the
+    // buffer has room for every request
+    const uint32_t* dcreated = exclusive_scan_u32_async(S.accepted.p, pos.p, m, c.prim, st);
+    RL_CUDA_TRY(cudaMemcpyAsync(c.read_slot() + kReadA, dcreated, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    const uint64_t need = G.num_new + m;
     if (need > G.new_tgt.n) {
         // grow, keeping what is already there
         DBuf<uint32_t> t2, s2;
         DBuf<int32_t> w2;
-        t2.alloc(need * 2);
-        s2.alloc(need * 2);
-        w2.alloc(need * 2);
+        const uint64_t room = need + need / 8;
+        t2.alloc(room);
+        s2.alloc(room);
+        w2.alloc(room);
         if (G.num_new) {
             RL_CUDA_TRY(cudaMemcpyAsync(t2.p, G.new_tgt.p, G.num_new * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
             RL_CUDA_TRY(cudaMemcpyAsync(s2.p, G.new_src.p, G.num_new * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
@@ -488,8 +492,11 @@ uint64_t run_connector(Ctx& c, uint32_t step, bool bind_axons) {
     k_emit_edges<<<blocks_for(m, 256), 256, 0, st>>>(m, S.accepted.p, pos.p, S.cidx.p, S.req_tgt.p, S.req_src.p, S.req_sig.p, G.num_new, G.new_tgt.p,
                                                      G.new_src.p, G.new_w.p);
     RL_LAUNCH_CHECK();
+    queue_error_read(c);
+    RL_CUDA_TRY(cudaStreamSynchronize(st));
+    const uint64_t created = c.read_slot()[kReadA];
     G.num_new += created;
-    check_device_error(c, "connector");
+    raise_device_error(c, "connector");
     c.stats.synapses_created += created;
     return created;
 }
@@ -689,16 +696,13 @@ uint64_t aggregate_edges(Ctx& c, bool count_only) {
     return kept;
 }
 
-uint64_t run_deletion(Ctx& c, uint32_t step, int type) {
+void queue_deletion(Ctx& c, uint32_t step, int type, unsigned long long* deleted) {
     Graph& G = c.graph;
     cudaStream_t st = c.stream;
-    rebuild_graph(c);
     if (G.num_edges == 0) {
         // nothing to delete: the elements say otherwise only if the state was set inconsistently
         RL_CUDA_TRY(cudaMemsetAsync(c.err.p, 0, sizeof(uint32_t), st));
     }
-    unsigned long long* d_cnt = reinterpret_cast<unsigned long long*>(c.counters.p) + 2;
-    RL_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), st));
     DeleteArgs A;
     A.n = c.n;
     A.type = type;
@@ -709,7 +713,7 @@ uint64_t run_deletion(Ctx& c, uint32_t step, int type) {
     A.signal = c.nr.signal.p;
     A.enabled = c.nr.enabled.p;
     A.in_off = G.offsets.p;
-    A.out_off = G.out_off.p;
+    A.out_off = G.num_edges ? G.out_off.p : G.offsets.p;  // without synapses every row is empty
     A.out_perm = G.out_perm.p;
     A.etgt = G.tgt.p;
     A.esrc = G.src.p;
@@ -718,24 +722,22 @@ uint64_t run_deletion(Ctx& c, uint32_t step, int type) {
         A.connected[t] = c.nr.connected[t].p;
         A.vacant[t] = c.nr.vacant[t].p;
     }
-    A.deleted = d_cnt;
+    A.deleted = deleted;
     A.err = c.err.p;
     k_delete<<<blocks_for(c.n, 128), 128, 0, st>>>(A);
     RL_LAUNCH_CHECK();
-    check_device_error(c, "synapse deletion");
-    unsigned long long deleted = 0;
-    RL_CUDA_TRY(cudaMemcpyAsync(&deleted, d_cnt, sizeof(deleted), cudaMemcpyDeviceToHost, st));
-    RL_CUDA_TRY(cudaStreamSynchronize(st));
+}
+
+void note_deleted(Ctx& c, uint64_t deleted) {
     // Entries whose weight reached zero stay until a rebuild drops them (once
     // they may be an eighth of the list): a zero entry adds nothing to a
     // neuron's input and is no synapse to a later deletion (a partner appears
     // |weight| times), and the edge order and both CSRs stay valid meanwhile;
     // rl_get_edges aggregates pairs and leaves zero weights out.
     if (deleted) {
-        G.zeros = true;
-        G.zero_bound += deleted;
+        c.graph.zeros = true;
+        c.graph.zero_bound += deleted;
     }
-    return deleted;
 }
 
 void bind_axons_host(Ctx& c, uint64_t m, const uint32_t* src) {

@@ -2054,19 +2054,6 @@ void launch_commit_f32(Ctx& c, int type, unsigned long long* total, const unsign
     RL_LAUNCH_CHECK();
 }
 
-uint64_t run_commit_f32(Ctx& c, int type) {
-    unsigned long long* d_del = reinterpret_cast<unsigned long long*>(c.counters.p) + 1;
-    RL_CUDA_TRY(cudaMemsetAsync(d_del, 0, sizeof(unsigned long long), c.stream));
-    k_commit_f32<<<blocks_for(c.n, 256), 256, 0, c.stream>>>(c.n, c.nr.enabled.p, c.nr.grown[type].p, c.nr.delta32[type].p, c.nr.connected[type].p,
-                                                             c.nr.vacant[type].p, c.cfg.retract_ratio[type], c.to_delete.p, d_del, nullptr, 0);
-    RL_LAUNCH_CHECK();
-    unsigned long long h = 0;
-    RL_CUDA_TRY(cudaMemcpyAsync(&h, d_del, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
-    RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
-    c.stats.bound_to_delete += h;
-    return h;
-}
-
 void pack_tree_f32(Ctx& c) {
     Tree& T = c.tree;
     if (T.recq_valid) {
@@ -2170,7 +2157,7 @@ void launch_search_wide_f32(Ctx& c, const uint32_t (&warps)[2], uint32_t segs0, 
         kern<<<blocks, WPB * 32, smem, c.stream>>>(B);
         RL_LAUNCH_CHECK();
     }
-    uint32_t left[4] = { 0, 0, 0, 0 };
+    uint32_t* left = c.read_slot() + kReadA;
     RL_CUDA_TRY(cudaMemcpyAsync(left, S.w_counts.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
     RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
     const uint64_t open = (uint64_t)left[0] + left[1];

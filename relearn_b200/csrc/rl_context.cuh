@@ -256,6 +256,11 @@ struct KernelParams {
     double cutoff = 0.0;
 };
 
+// Counts of an update (Ctx::commit_cnt), and the pinned words behind their host copy.
+constexpr size_t kCommitCounts = 10;
+constexpr size_t kReadSlot = 12;
+constexpr int kReadError = 0, kReadA = 1, kReadB = 2;
+
 struct Ctx;
 // Records an event pair around a scope when profiling is on.
 struct PhaseScope {
@@ -380,8 +385,13 @@ struct Ctx {
     DBuf<uint32_t> to_delete;  // per neuron, bound elements to delete in the current pass
     DBuf<uint32_t> err;       // device error word
     DBuf<uint64_t> counters;  // device counters
-    DBuf<unsigned long long> commit_cnt;  // bound elements to delete per element type of an update, then vacant axons
-    unsigned long long* h_commit = nullptr;  // pinned host copy of commit_cnt (read without blocking the enqueue)
+    // an update's counts: bound elements to delete per element type (0-2) and
+    // vacant axons (3) of the commits in one launch, bound elements of the
+    // commits behind deletions (4-6), deleted synapses (7-9)
+    DBuf<unsigned long long> commit_cnt;
+    unsigned long long* h_commit = nullptr;  // pinned host copy of commit_cnt (read without blocking the enqueue), then the words of read_slot
+    uint32_t* read_slot() const;             // pinned words for small reads (kRead*)
+    cudaEvent_t commit_read = nullptr;       // the counts of an update's deletions have landed
     bool target_uniform = true;  // every neuron has cfg.target_calcium as its target
     // Host transfers that overlap the work on the context's stream: uploads
     // of enabled flags and snapshots of calcium and fired flags go through
@@ -474,7 +484,8 @@ uint64_t run_connector(Ctx& c, uint32_t step, bool bind_axons = true);
 void bind_axons_host(Ctx& c, uint64_t m, const uint32_t* src);  // one vacant axon per listed source
 void rebuild_graph(Ctx& c);                     // merge new edges into the CSR
 uint64_t aggregate_edges(Ctx& c, bool count_only);  // the list rl_get_edges returns, in graph.m_tgt, m_src, m_w
-uint64_t run_deletion(Ctx& c, uint32_t step, int type);  // delete to_delete[] synapses per neuron for one element type
+void queue_deletion(Ctx& c, uint32_t step, int type, unsigned long long* deleted);  // delete to_delete[] synapses per neuron for one element type
+void note_deleted(Ctx& c, uint64_t deleted);                                        // the host's share of it, once the count is read
 void add_edges_host(Ctx& c, uint64_t m, const uint32_t* t, const uint32_t* s, const int32_t* w);
 
 // fp32.cu (precision form)
@@ -490,7 +501,6 @@ void launch_activity_f32_steps(Ctx& c, uint32_t nsteps);
 void launch_activity_fp64_steps(Ctx& c, uint32_t nsteps);
 bool launch_activity_f32_coupled(Ctx& c, uint32_t nsteps);
 bool launch_activity_fp64_coupled(Ctx& c, uint32_t nsteps);
-uint64_t run_commit_f32(Ctx& c, int type);
 void pack_tree_f32(Ctx& c);
 void launch_search_f32(Ctx& c, int type, const uint32_t* seg_warp, const uint64_t* seg_begin, const uint64_t* seg_end, const uint32_t* seg_net,
                        uint32_t num_segs, uint32_t warps, uint32_t step, const SearchVariant& v, uint32_t* tasks);
@@ -509,7 +519,7 @@ void ensure_copy_stream(Ctx& c);
 // the next work has been queued on the context's stream, so that the copies
 // overlap it (and do not hold up an upload issued in between).
 void issue_snapshots(Ctx& c);
-uint64_t run_commit(Ctx& c, int type);
+void queue_commit(Ctx& c, int type, unsigned long long* bound);
 // Commit of `type` that does nothing when an earlier type of the same update
 // (its count in commit_cnt) left bound elements to delete; counts into
 // commit_cnt[type].  The three are launched back to back and read once.
@@ -522,5 +532,7 @@ void launch_vacant_axon_count(Ctx& c, unsigned long long* out);
 void launch_commit_f32(Ctx& c, int type, unsigned long long* total, const unsigned long long* guard, int guard_n);  // commit one element type; to_delete[] per neuron, returns the sum
 
 void check_device_error(Ctx& c, const char* phase);
+void queue_error_read(Ctx& c);                        // the same in two parts: copy the error word ...
+void raise_device_error(Ctx& c, const char* phase);   // ... and, after a synchronisation, throw if it is set
 
 }  // namespace rl
