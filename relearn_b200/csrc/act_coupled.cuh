@@ -17,6 +17,10 @@
 // cluster barrier (6,100 neurons: 3.4 us per step FP64, 2.6 FP32); more are
 // launched cooperatively (the launch fails rather than leave one of them out)
 // and count arrivals in device memory (6,200 neurons: 3.7 and 3.1 us).
+// More neurons than resident threads run in rounds, several per thread with
+// their state in shared memory (up to 1,136,640 neurons FP64, 1,875,456 FP32;
+// untuned launch per step -> here: FP64 171,000 neurons 12.8 -> 8.8, 500,000
+// 21.2 -> 19.0, 1M 38.0 -> 33.7; FP32 7.1 -> 5.2, 12.6 -> 8.5, 21.5 -> 14.4).
 #pragma once
 
 #include "rl_context.cuh"
@@ -25,6 +29,7 @@ namespace rl {
 
 constexpr int kCoupledBlock = 384;          // threads (neurons) per block, two blocks per SM
 constexpr unsigned kCoupledCluster = 16;    // blocks per cluster (8 are portable)
+constexpr uint32_t kCoupledChunk = 16;      // steps between two replays of calcium and growth (bits of a uint16_t)
 constexpr uint32_t kCoupledPolls = 1u << 22;  // polls of a barrier before it gives up: some seconds
 
 #if defined(__CUDACC__)
@@ -107,6 +112,38 @@ __device__ __forceinline__ void push_warp(bool f, uint32_t o0, uint32_t o1, cons
     }
     __syncwarp();
 }
+
+// The block's queued spikes (neurons base + who[q]), eight lanes each.
+template <int BLOCK, typename T>
+__device__ __forceinline__ void push_queue(uint32_t cnt, uint32_t base, const uint16_t* who, const uint32_t* __restrict__ out_off,
+                                           const uint32_t* __restrict__ out_perm, const uint32_t* __restrict__ tgt, const int32_t* __restrict__ w,
+                                           T* next) {
+    for (uint32_t q = threadIdx.x >> 3; q < cnt; q += BLOCK / 8) {
+        const uint32_t i = base + who[q];
+        const uint32_t o1 = out_off[i + 1];
+        for (uint32_t j = out_off[i] + (threadIdx.x & 7u); j < o1; j += 8u) {
+            const uint32_t e = out_perm[j];
+            add_weight(next + tgt[e], w[e]);
+        }
+    }
+}
+
+// Appends `slot` of the lanes with `take` set to the queue.  All lanes call it.
+__device__ __forceinline__ void queue_slots(bool take, uint32_t slot, uint16_t* who, uint32_t* cnt) {
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, take);
+    if (mask == 0u) {
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t first = 0;
+    if (lane == 0) {
+        first = atomicAdd(cnt, (uint32_t)__popc(mask));
+    }
+    first = __shfl_sync(0xFFFFFFFFu, first, 0);
+    if (take) {
+        who[first + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = (uint16_t)slot;
+    }
+}
 #endif
 
 // Launches the coupled kernel of `steps` steps (its cluster form for few blocks) if all its
@@ -144,6 +181,46 @@ bool launch_coupled(Ctx& c, uint32_t steps, void (*cluster_kernel)(KArgs...), vo
     PhaseScope ps(c, PH_ACTIVITY_KERNEL, steps);
     if (cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...) != cudaSuccess) {
         (void)cudaGetLastError();  // such a launch is not available here: the caller takes one launch per step
+        return false;
+    }
+    if (g_bind.launches) {
+        ++*g_bind.launches;
+    }
+    return true;
+}
+
+// The form for more neurons than resident threads: `rounds` neurons per
+// thread, their x, u and draws in shared memory (`bytes` per neuron), at most
+// `per_sm_target` blocks per SM; false where they do not all fit.
+template <typename Args>
+bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, uint32_t*, uint32_t*),
+                           unsigned per_sm_target, size_t bytes, const Args& args, uint8_t* fired_before_last) {
+    const unsigned slots = per_sm_target * (unsigned)c.num_sms;
+    const uint32_t rounds = blocks_for(c.n, slots * kCoupledBlock);
+    const unsigned blocks = blocks_for(c.n, rounds * kCoupledBlock);
+    const size_t smem = bytes * rounds * kCoupledBlock;
+    if (rounds * kCoupledBlock > 65536u || smem > (size_t)c.smem_optin - 1024) {
+        return false;
+    }
+    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, kCoupledBlock, smem));
+    if (blocks > (unsigned)per_sm * (unsigned)c.num_sms) {
+        return false;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kCoupledBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PhaseScope ps(c, PH_ACTIVITY_KERNEL, steps);
+    if (cudaLaunchKernelEx(&cfg, kernel, args, (const ActDesc*)c.act_desc.p, steps, rounds, fired_before_last, c.act_bar.p, c.err.p) != cudaSuccess) {
+        (void)cudaGetLastError();
         return false;
     }
     if (g_bind.launches) {

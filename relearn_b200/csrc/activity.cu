@@ -914,6 +914,186 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled(ActArgs
     }
 }
 
+// The same for more neurons than resident threads: a thread steps `rounds`
+// neurons (block slots r * BLOCK + threadIdx.x), whose x, u and next draw stay
+// in shared memory.  The draws of the next step and, every kCoupledChunk steps,
+// calcium and growth (from the chunk's spike bits, k_calcium_growth's
+// operations in its order) fill the time between arriving at the barrier and
+// its completion.
+constexpr size_t kRounds64Bytes = 3 * sizeof(double) + 2 * sizeof(uint16_t) + 1;
+
+template <int BLOCK, int H, int MODEL, bool TOP>
+__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled_rounds(ActArgs A, const ActDesc* __restrict__ D, uint32_t nsteps,
+                                                                                uint32_t rounds, uint8_t* __restrict__ fired_before_last,
+                                                                                uint32_t* bar, uint32_t* err) {
+    extern __shared__ double s_dyn64[];
+    __shared__ uint32_t s_cnt[2];  // queued tail draws, queued spikes
+    const uint32_t per = rounds * BLOCK;
+    double* s_x = s_dyn64;
+    double* s_u = s_x + per;
+    double* s_z = s_u + per;
+    uint16_t* s_who = reinterpret_cast<uint16_t*>(s_z + per);  // either queue: a block barrier lies between their uses
+    uint16_t* s_hist = s_who + per;                            // spike flags of the chunk's steps
+    uint8_t* s_flag = reinterpret_cast<uint8_t*>(s_hist + per);  // bit 0: enabled, bit 1: spike flag
+    const uint32_t base = blockIdx.x * per;
+    const uint32_t step0 = D->base_step;
+    const uint32_t* __restrict__ out_off = D->out_off;
+    const uint32_t* __restrict__ out_perm = D->out_perm;
+    const uint32_t* __restrict__ tgt_of = D->tgt;
+    const int32_t* __restrict__ w_of = D->w;
+    const Nu nu{ { A.nu1[0], A.nu1[1], A.nu1[2] } };
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+        uint8_t flag = 0;
+        if (i < A.n) {
+            flag = (uint8_t)((A.enabled[i] ? 1u : 0u) | (A.fired_prev[i] ? 2u : 0u));
+            s_x[s] = A.x[i];
+            s_u[s] = A.u[i];
+        }
+        s_flag[s] = flag;
+        s_hist[s] = 0;
+    }
+    if (threadIdx.x < 2) {
+        s_cnt[threadIdx.x] = 0u;
+    }
+    __syncthreads();
+    auto draws = [&](uint32_t step) {
+        const uint32_t odd = threadIdx.x & 1u;
+        for (uint32_t r = 0; r < rounds; r += 2u) {
+            // lane pairs hold neuron pairs: the even lane computes round r's
+            // Philox block, the odd lane round r + 1's, and they swap words
+            const u32x4 b = noise_block_rk(A.rk0, A.rk1, step, base + (r + odd) * BLOCK + threadIdx.x);
+            const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? b.x : b.z, 1);
+            const uint32_t g1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? b.y : b.w, 1);
+            const uint64_t got = ((uint64_t)g0 << 21) | (uint64_t)(g1 >> 11);
+            const uint64_t bits[2] = { odd ? got : (((uint64_t)b.x << 21) | (uint64_t)(b.y >> 11)),
+                                       odd ? (((uint64_t)b.z << 21) | (uint64_t)(b.w >> 11)) : got };
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; ++h) {
+                if (r + h < rounds) {
+                    const uint32_t s = (r + h) * BLOCK + threadIdx.x;
+                    const bool use = (s_flag[s] & 1u) != 0u;
+                    const double p = uniform_from_bits53(bits[h]);
+                    const bool tail = use && normal_in_tail(p);
+                    queue_slots(tail, s, s_who, &s_cnt[0]);
+                    s_z[s] = tail ? p : (use ? normal_quantile_central(p) : 0.0);
+                }
+            }
+        }
+        __syncthreads();
+        const uint32_t cnt = s_cnt[0];
+        for (uint32_t q = threadIdx.x; q < cnt; q += BLOCK) {
+            const uint32_t s = s_who[q];
+            s_z[s] = normal_quantile_tail(s_z[s]);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_cnt[0] = 0u;  // next used behind the barrier of the step
+        }
+    };
+    draws(step0);
+    for (uint32_t k = 0; k < nsteps; ++k) {
+        const uint32_t step = step0 + k;
+        const bool last = k + 1 == nsteps;
+        if (k > 0 && !step_wait<false>(bar, k * gridDim.x, err)) {
+            return;
+        }
+        long long* in = A.syn_in[step & 1u];
+        const uint32_t bit = k % kCoupledChunk;
+        long long next = k > 0 && base + threadIdx.x < A.n ? __ldcg(in + base + threadIdx.x) : 0;
+        for (uint32_t r = 0; r < rounds; ++r) {
+            const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+            long long isum = next;
+            next = k > 0 && r + 1 < rounds && i + BLOCK < A.n ? __ldcg(in + i + BLOCK) : 0;
+            const uint32_t flag = s_flag[s];
+            const bool on = (flag & 1u) != 0u;
+            bool f = (flag & 2u) != 0u;
+            if (isum != 0) {
+                __stcg(in + i, 0ll);
+            }
+            if (k == 0 && on) {
+                isum = synaptic_sum(A, D, i);
+            }
+            if (on) {
+                const double input = step_input(A, isum, s_z[s]);
+                double xv = s_x[s], uv = s_u[s];
+                if constexpr (MODEL == RL_MODEL_IZHIKEVICH && H > 0) {
+                    f = izhikevich_frozen<H, TOP>(A, input, xv, uv) != 0;
+                } else {
+                    f = model_step<H, MODEL>(A, step, A.seed1, i, input, xv, uv) != 0;
+                }
+                s_x[s] = xv;
+                s_u[s] = uv;
+                s_flag[s] = (uint8_t)(1u | (f ? 2u : 0u));
+                s_hist[s] = (uint16_t)((bit ? s_hist[s] : 0u) | ((f ? 1u : 0u) << bit));
+                if (last && A.input) {
+                    A.input[i] = input;
+                }
+            } else if (last && A.input && i < A.n) {
+                A.input[i] = 0.0;
+            }
+            if (i < A.n && k + 2 >= nsteps) {
+                (last ? A.fired_cur : fired_before_last)[i] = f ? 1 : 0;
+            }
+            __syncwarp();
+            if (!last) {
+                queue_slots(f, s, s_who, &s_cnt[1]);  // a disabled neuron keeps its flag, and its targets read it
+            }
+        }
+        if (!last) {
+            __syncthreads();
+            push_queue<BLOCK>(s_cnt[1], base, s_who, out_off, out_perm, tgt_of, w_of, A.syn_in[(step + 1u) & 1u]);
+            step_arrive<false>(bar);
+            if (threadIdx.x == 0) {
+                s_cnt[1] = 0u;  // read by all before the arrival's block barrier
+            }
+            draws(step + 1u);
+        }
+        if (bit + 1u == kCoupledChunk || last) {
+            for (uint32_t r = 0; r < rounds; ++r) {
+                const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+                if ((s_flag[s] & 1u) != 0u) {
+                    double ca = A.calcium[i], d0 = A.delta0[i], d1 = A.delta1[i], d2 = A.delta2[i];
+                    const uint32_t spikes = s_hist[s];
+                    bool flat = false;
+                    if constexpr (H > 0) {
+                        if (A.uniform_target) {
+                            for (uint32_t j = 0; j <= bit; ++j) {
+                                calcium_growth_flat<H, false>(A, (uint8_t)((spikes >> j) & 1u), nu, ca, d0, d1, d2);
+                            }
+                            flat = true;
+                        }
+                    }
+                    if (!flat) {
+                        const double tgt = A.uniform_target ? 0.0 : A.target[i];
+                        for (uint32_t j = 0; j <= bit; ++j) {
+                            ca = calcium_step<H>(A, (uint8_t)((spikes >> j) & 1u), ca);
+                            d0 = d0 + growth_step(A, 0, ca, tgt, nu);
+                            d1 = d1 + growth_step(A, 1, ca, tgt, nu);
+                            d2 = d2 + growth_step(A, 2, ca, tgt, nu);
+                        }
+                    }
+                    A.calcium[i] = ca;
+                    A.delta0[i] = d0;
+                    A.delta1[i] = d1;
+                    A.delta2[i] = d2;
+                } else if (last && i < A.n) {
+                    A.delta0[i] = A.delta0[i] + 0.0;
+                    A.delta1[i] = A.delta1[i] + 0.0;
+                    A.delta2[i] = A.delta2[i] + 0.0;
+                }
+            }
+        }
+    }
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+        if ((s_flag[s] & 1u) != 0u) {
+            A.x[i] = s_x[s];
+            A.u[i] = s_u[s];
+        }
+    }
+}
+
 struct CommitArgs {
     uint32_t n;
     const uint8_t* enabled;
@@ -1219,7 +1399,9 @@ void launch_calcium_growth64(Ctx& c, uint32_t row0, uint32_t m, cudaStream_t st)
 template <int H, int MODEL, bool TOP = false>
 bool launch_coupled64_m(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_before_last) {
     return launch_coupled(c, nsteps, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, true>, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, false>, A,
-                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p);
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p) ||
+           launch_coupled_rounds(c, nsteps, &k_activity_coupled_rounds<kCoupledBlock, H, MODEL, TOP>, 768 / kCoupledBlock, kRounds64Bytes, A,
+                                 fired_before_last);
 }
 
 template <int H>

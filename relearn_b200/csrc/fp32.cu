@@ -696,6 +696,143 @@ __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled(Ac
     }
 }
 
+// The same for more neurons than resident threads: a thread steps `rounds`
+// neurons (block slots r * BLOCK + threadIdx.x), whose x, u and next draw stay
+// in shared memory; calcium and growth are replayed from the spike bits every
+// kCoupledChunk steps (k_calcium_growth_f32's operations in its order).
+constexpr size_t kRounds32Bytes = 3 * sizeof(float) + 2 * sizeof(uint16_t) + 1;
+
+template <int BLOCK, int H, int MODEL>
+__global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled_rounds(Act32 A, const ActDesc* __restrict__ D, uint32_t nsteps,
+                                                                                    uint32_t rounds, uint8_t* __restrict__ fired_before_last,
+                                                                                    uint32_t* bar, uint32_t* err) {
+    extern __shared__ float s_dyn32[];
+    __shared__ uint32_t s_cnt;  // queued spikes
+    const uint32_t per = rounds * BLOCK;
+    float* s_x = s_dyn32;
+    float* s_u = s_x + per;
+    uint32_t* s_word = reinterpret_cast<uint32_t*>(s_u + per);
+    uint16_t* s_who = reinterpret_cast<uint16_t*>(s_word + per);
+    uint16_t* s_hist = s_who + per;
+    uint8_t* s_flag = reinterpret_cast<uint8_t*>(s_hist + per);  // bit 0: enabled, bit 1: spike flag
+    const uint32_t base = blockIdx.x * per;
+    const uint32_t step0 = D->base_step;
+    const uint32_t* __restrict__ out_off = D->out_off;
+    const uint32_t* __restrict__ out_perm = D->out_perm;
+    const uint32_t* __restrict__ tgt_of = D->tgt;
+    const int32_t* __restrict__ w_of = D->w;
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+        uint8_t flag = 0;
+        float x = 0.0f, u = 0.0f;
+        if (i < A.n) {
+            flag = (uint8_t)((A.enabled[i] ? 1u : 0u) | (A.fired_prev[i] ? 2u : 0u));
+            x = A.x[i];
+            u = A.u[i];
+        }
+        s_x[s] = x;
+        s_u[s] = u;
+        s_flag[s] = flag;
+        s_hist[s] = 0;
+    }
+    if (threadIdx.x == 0) {
+        s_cnt = 0u;
+    }
+    __syncthreads();
+    auto draws = [&](uint32_t step) {
+        const uint32_t odd = threadIdx.x & 1u;
+        for (uint32_t r = 0; r < rounds; r += 2u) {
+            const u32x4 b = noise_block_rk(A.rk0, A.rk1, step, base + (r + odd) * BLOCK + threadIdx.x);
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? b.x : b.z, 1);
+            s_word[r * BLOCK + threadIdx.x] = odd ? got : b.x;
+            if (r + 1u < rounds) {
+                s_word[(r + 1u) * BLOCK + threadIdx.x] = odd ? b.z : got;
+            }
+        }
+    };
+    draws(step0);
+    for (uint32_t k = 0; k < nsteps; ++k) {
+        const uint32_t step = step0 + k;
+        const bool last = k + 1 == nsteps;
+        if (k > 0 && !step_wait<false>(bar, k * gridDim.x, err)) {
+            return;
+        }
+        int32_t* in = A.syn_in[step & 1u];
+        const uint32_t bit = k % kCoupledChunk;
+        int32_t next = k > 0 && base + threadIdx.x < A.n ? __ldcg(in + base + threadIdx.x) : 0;
+        for (uint32_t r = 0; r < rounds; ++r) {
+            const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+            const int32_t pushed = next;
+            next = k > 0 && r + 1 < rounds && i + BLOCK < A.n ? __ldcg(in + i + BLOCK) : 0;
+            const uint32_t flag = s_flag[s];
+            const bool on = (flag & 1u) != 0u;
+            if (pushed != 0) {
+                __stcg(in + i, 0);
+            }
+            uint32_t k24p = 0;
+            if (MODEL == RL_MODEL_POISSON) {
+                k24p = philox4x32_10_rk(u32x4{ step, i, 0u, (uint32_t)STREAM_POISSON << 24 }, A.rk0, A.rk1).x >> 8;
+            }
+            float x = s_x[s], u = s_u[s], input, d[3] = { 0.0f, 0.0f, 0.0f };
+            double ca = 0.0;
+            const Grow32 G{};
+            uint8_t f;
+            neuron_f32<H, MODEL, true, false>(A, D, i, on, (uint8_t)((flag >> 1) & 1u), s_word[s] >> 8, k24p, A.nu1, G, x, u, ca, d, input, f, k == 0,
+                                              pushed);
+            if (on) {
+                s_x[s] = x;
+                s_u[s] = u;
+                s_flag[s] = (uint8_t)(1u | (f ? 2u : 0u));
+                s_hist[s] = (uint16_t)((bit ? s_hist[s] : 0u) | ((f ? 1u : 0u) << bit));
+            }
+            if (i < A.n && k + 2 >= nsteps) {
+                (last ? A.fired_cur : fired_before_last)[i] = f ? 1 : 0;
+                if (last && A.input) {
+                    A.input[i] = input;
+                }
+            }
+            __syncwarp();
+            if (!last) {
+                queue_slots(f != 0, s, s_who, &s_cnt);  // a disabled neuron keeps its flag, and its targets read it
+            }
+        }
+        if (!last) {
+            __syncthreads();
+            push_queue<BLOCK>(s_cnt, base, s_who, out_off, out_perm, tgt_of, w_of, A.syn_in[(step + 1u) & 1u]);
+            step_arrive<false>(bar);
+            if (threadIdx.x == 0) {
+                s_cnt = 0u;  // read by all before the arrival's block barrier; next used behind the step's
+            }
+            draws(step + 1u);
+        }
+        if (bit + 1u == kCoupledChunk || last) {
+            for (uint32_t r = 0; r < rounds; ++r) {
+                const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+                if ((s_flag[s] & 1u) != 0u) {
+                    const Grow32 G = grow32_of(A, A.target ? A.target[i] : 0.0f);
+                    double ca = A.calcium[i];
+                    float d[3] = { A.delta[0][i], A.delta[1][i], A.delta[2][i] };
+                    const uint32_t spikes = s_hist[s];
+                    for (uint32_t j = 0; j <= bit; ++j) {
+                        calcium_growth_f32(A, (uint8_t)((spikes >> j) & 1u), A.nu1, G, ca, d);
+                    }
+                    A.calcium[i] = ca;
+                    A.delta[0][i] = d[0];
+                    A.delta[1][i] = d[1];
+                    A.delta[2][i] = d[2];
+                }
+            }
+        }
+    }
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t s = r * BLOCK + threadIdx.x, i = base + s;
+        if ((s_flag[s] & 1u) != 0u) {
+            A.x[i] = s_x[s];
+            A.u[i] = s_u[s];
+        }
+    }
+}
+
 // Two FP32 values in one 64-bit register pair; each operation rounds both
 // halves as the scalar instruction does (fma.rn.f32x2 and its kin issue once
 // for two lanes' worth of arithmetic).
@@ -1994,7 +2131,9 @@ namespace {
 template <int H, int MODEL>
 bool launch_coupled32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_before_last) {
     return launch_coupled(c, nsteps, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, true>, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, false>, A,
-                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p);
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p) ||
+           launch_coupled_rounds(c, nsteps, &k_activity_f32_coupled_rounds<kCoupledBlock, H, MODEL>, 1152 / kCoupledBlock, kRounds32Bytes, A,
+                                 fired_before_last);
 }
 
 }  // namespace

@@ -1,7 +1,7 @@
 """A block of activity steps of a network with synapses in one launch gives the
 bits of one launch per step: at the edges of its forms (a cluster of up to
-sixteen blocks of 384 neurons, a resident grid of more, one launch per step where
-the neurons outnumber the resident threads), both precision forms, every neuron
+sixteen blocks of 384 neurons, a resident grid of more, several neurons per
+thread, one launch per step where even those do not hold the network), both precision forms, every neuron
 model, disabled neurons that keep a set spike flag, targets of their own, other
 substep counts, and blocks of even and odd length that follow each other."""
 import numpy as np
@@ -46,7 +46,8 @@ def state(net):
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("n,model,h", [(2, 0, 10), (383, 0, 10), (384, 0, 7), (385, 1, 10), (3073, 0, 10), (6144, 0, 10), (6145, 0, 10), (6145, 3, 10), (6144, 3, 10),
                                        (20011, 0, 10), (20012, 0, 10), (20011, 2, 10), (20012, 1, 10), (113664, 0, 10), (113665, 0, 10),
-                                       (170496, 0, 10), (170497, 0, 10)])
+                                       (170496, 0, 10), (170497, 0, 10), (180001, 3, 10), (180002, 1, 10), (180003, 2, 10), (180004, 0, 7),
+                                       (400003, 0, 10), (1136640, 0, 10), (1136641, 0, 10)])
 def test_coupled_block_equals_steps(n, model, h, precision):
     nets = [make(n, precision, model, fused, h) for fused in (False, True)]
     spikes = 0
