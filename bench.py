@@ -231,18 +231,23 @@ CAPTURED = {
     # the fused block kernels (a network without synapses: a block of steps per
     # launch, state in registers), from the instruction mix of one 100-step
     # launch at 1M neurons (bench.py --case activity --case-steps 100), per
-    # neuron-step: k_activity_steps 10.08 FP64 warp instructions (DMUL 3.80,
-    # DADD 3.55, DFMA 1.82, DSETP 0.92); k_activity_f32_steps 5.85 warp
+    # neuron-step: k_activity_steps 9.05 warp instructions on the FP64 pipe;
+    # k_activity_f32_pairs 5.10 warp
     # instructions of every kind, issued at one per SM sub-partition (4 per
     # SM) per cycle; DRAM read + write of that launch
-    "fused64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "e6ef1fe863ecbbd9", "fp64_warp_instr_per_neuron": 10.08,
-                "traffic": 50.06e6 + 4.06e6},
-    "fused32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "ae16ba4013f08c25", "warp_instr_per_neuron": 5.85, "traffic": 30.02e6 + 0.14e6},
+    "fused64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "83fc480b4074af9a", "fp64_warp_instr_per_neuron": 9.05,
+                "traffic": 50.07e6 + 3.76e6},
+    "fused32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "66ca8356202a8dc8", "warp_instr_per_neuron": 5.10, "traffic": 30.02e6 + 0.19e6},
     # the batched block kernel over the 128-network configuration (7.15M
     # neurons, bench.py --case ensemble --case-steps 100 --precision fp32):
     # warp instructions per neuron-step, DRAM read + write of the launch
     "ensemble32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "ae16ba4013f08c25", "warp_instr_per_neuron": 5.95,
                    "traffic": 215.10e6 + 187.94e6},
+    # a coupled block of 100 steps at 1M neurons with two synapses each, per
+    # neuron-step: FP32 warp instructions of every kind (k_activity_f32_coupled_rounds);
+    # FP64: the block kernel's, whose FP64 functions it runs
+    "coupled64": {"sources": ("act_coupled.cuh", "activity.cu", "rl_math.cuh"), "digest": "dfefc858881614f5", "fp64_warp_instr_per_neuron": 9.05},
+    "coupled32": {"sources": ("act_coupled.cuh", "fp32.cu", "rl_math.cuh"), "digest": "1c0a356d44151c38", "warp_instr_per_neuron": 9.58},
     # the search snapshot at 1M (bench.py --case search; the excitatory pass,
     # 0.8M searches): lanes active per warp instruction, L1 / L2 hit rates of
     # the walk, DRAM bytes per search
@@ -312,7 +317,7 @@ def fused_roofline(precision: int, n: int, step_us: float, act_cnt: int, sm_mhz,
     else:
         achieved = cap["warp_instr_per_neuron"] * n / (step_us * 1e-6) / 1e12
         peak = 4 * B200_SMS * mhz * 1e6 / 1e12
-        roof = {"bound": "issue", "kernel": "k_activity_f32_steps", "achieved": achieved, "peak": peak, "unit": "T warp-inst/s",
+        roof = {"bound": "issue", "kernel": "k_activity_f32_pairs", "achieved": achieved, "peak": peak, "unit": "T warp-inst/s",
                 "frac": achieved / peak, "warp_instr_per_neuron_step": cap["warp_instr_per_neuron"],
                 "peak_kind": "nominal issue rate at the median SM clock: 1 warp instruction per SM sub-partition per cycle x 592"}
     bytes_per_launch = FUSED_BYTES[precision] * n
@@ -324,13 +329,13 @@ def fused_roofline(precision: int, n: int, step_us: float, act_cnt: int, sm_mhz,
     return roof
 
 
-def step_compute(precision: int, n: int, step_us: float, sm_mhz=None) -> dict:
-    """The compute side of one launch per step (step kernel + the chunk's
-    calcium and growth) from the captured instruction counts: FP64 lane
-    operations against the FP64 pipe (FP64 form), warp instructions against
-    the issue rate (FP32 form)."""
+def step_compute(precision: int, n: int, step_us: float, sm_mhz=None, coupled: bool = False) -> dict:
+    """The compute side of a step with synapses (one launch per step with the
+    chunk's calcium and growth, or a coupled block of steps in one launch) from
+    the captured instruction counts: FP64 lane operations against the FP64 pipe
+    (FP64 form), warp instructions against the issue rate (FP32 form)."""
     mhz = sm_mhz or 1965.0
-    cap = captured("activity64" if precision == 0 else "activity32")
+    cap = captured(("coupled" if coupled else "activity") + ("64" if precision == 0 else "32"))
     if precision == 0:
         lane_ops = cap["fp64_warp_instr_per_neuron"] * 32
         achieved = lane_ops * n / (step_us * 1e-6) / 1e12
@@ -660,15 +665,17 @@ def synapse_regime(args, dev, stream, world, precision):
     per_neuron = ACT_BYTES_PER_NEURON if precision == 0 else ACT_BYTES_FP32
     bytes_per_launch = step_bytes(precision, n, edges)
     act_achieved = bytes_per_launch / (act_ms / act_cnt / 1e3) / 1e9 if act_cnt else 0.0
-    act_roof = {"bound": "hbm", "kernel": "k_activity" if precision == 0 else "k_activity_f32", "achieved": act_achieved, "peak": hbm,
+    act_roof = {"bound": "hbm", "kernel": ("k_activity" if precision == 0 else "k_activity_f32") + ("_coupled_rounds" if args.step_fusion else ""), "achieved": act_achieved, "peak": hbm,
                 "unit": "GB/s", "frac": act_achieved / hbm, "peak_kind": peak_kind, "bytes_per_launch": bytes_per_launch,
                 "avg_launch_us": 1e3 * act_ms / act_cnt if act_cnt else None, "launches": act_cnt,
                 "bytes": f"{per_neuron:.2f} B per neuron-step + {ACT_BYTES_PUSHED[precision]} B pushed sum per neuron-step + per 100-step block "
                          f"{ACT_BYTES_CSR_ROW} B row offsets per neuron and {ACT_BYTES_PER_EDGE} B per in-edge",
-                "kernels": "the step kernel (k_activity / k_activity_f32, one launch per step) and the chunks' calcium and growth (k_calcium_growth / "
+                "kernels": "k_activity_coupled / k_activity_f32_coupled (_rounds): a block of steps in one launch, the state on chip between its steps; "
+                           "the bytes are those of one launch per step" if args.step_fusion else
+                           "the step kernel (k_activity / k_activity_f32, one launch per step) and the chunks' calcium and growth (k_calcium_growth / "
                            "k_calcium_growth_f32, one launch per chunk of up to 64 steps)"}
     if act_cnt:
-        comp = step_compute(precision, n, 1e3 * act_ms / act_cnt)
+        comp = step_compute(precision, n, 1e3 * act_ms / act_cnt, coupled=bool(args.step_fusion))
         act_roof["compute"] = comp
         if comp["frac"] > act_roof["frac"]:
             # the arithmetic side is the nearer bound: report it first
