@@ -199,10 +199,11 @@ bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const Ac
     const uint32_t rounds = blocks_for(c.n, slots * kCoupledBlock);
     const unsigned blocks = blocks_for(c.n, rounds * kCoupledBlock);
     const size_t smem = bytes * rounds * kCoupledBlock;
-    if (rounds * kCoupledBlock > 65536u || smem > (size_t)c.smem_optin - 1024) {
+    constexpr size_t kFixed = 1024;  // at least the kernels' static shared memory
+    if (rounds * kCoupledBlock > 65536u || smem > (size_t)c.smem_optin - kFixed) {
         return false;
     }
-    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared_memory(c, kernel, kFixed);
     int per_sm = 0;
     RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, kCoupledBlock, smem));
     if (blocks > (unsigned)per_sm * (unsigned)c.num_sms) {

@@ -973,7 +973,7 @@ void launch_bins_kernel(Ctx& c, const BinsArgs& A) {
     constexpr int WPB = 4;
     auto kern = &k_search_bins<WPB, SQUARED>;
     const size_t smem = 64 * sizeof(double) + WPB * bins_warp_bytes(A.levels);
-    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared_memory(c, kern);
     int per_sm = 0;
     RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kern, WPB * 32, smem));
     const uint32_t tasks = A.num_tasks[0] + A.num_tasks[1];
@@ -1291,7 +1291,7 @@ void run_search(Ctx& c, uint32_t step) {
                     const HotKernel kern = fp64_hot_kernel(v);
                     const uint32_t hot = hot_nodes(c, v, sizeof(double4) + sizeof(uint4) + sizeof(double));
                     const size_t smem = (size_t)hot * (sizeof(double4) + sizeof(uint4) + sizeof(double));
-                    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    allow_shared_memory(c, kern);
                     const unsigned blocks = std::min<unsigned>((unsigned)c.num_sms, (launches[t].warps + 31) / 32);
                     kern<<<blocks, 1024, smem, st>>>(args[t], hot);
                     RL_LAUNCH_CHECK();

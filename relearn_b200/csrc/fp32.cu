@@ -2248,7 +2248,7 @@ void launch_search_f32(Ctx& c, int type, const uint32_t* seg_warp, const uint64_
         const auto kern = v.packet == 16 ? &k_search_f32_hot<16> : &k_search_f32_hot<32>;
         const uint32_t hot = hot_nodes(c, v, 2 * sizeof(uint4));
         const size_t smem = (size_t)hot * 2 * sizeof(uint4);
-        RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(c, kern);
         const unsigned blocks = std::min<unsigned>((unsigned)c.num_sms, (warps + 31) / 32);
         kern<<<blocks, 1024, smem, c.stream>>>(A, hot);
         RL_LAUNCH_CHECK();
@@ -2288,7 +2288,7 @@ void launch_search_wide_f32(Ctx& c, const uint32_t (&warps)[2], uint32_t segs0, 
     {
         auto kern = c.kernel.type == RL_KERNEL_GAUSSIAN ? &k_search_bins32<WPB, true> : &k_search_bins32<WPB, false>;
         const size_t smem = WPB * bins_warp_bytes(B.levels);
-        RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(c, kern);
         int per_sm = 0;
         RL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kern, WPB * 32, smem));
         const uint32_t tasks = B.num_tasks[0] + B.num_tasks[1];

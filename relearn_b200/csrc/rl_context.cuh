@@ -488,6 +488,16 @@ void queue_deletion(Ctx& c, uint32_t step, int type, unsigned long long* deleted
 void note_deleted(Ctx& c, uint64_t deleted);                                        // the host's share of it, once the count is read
 void add_edges_host(Ctx& c, uint64_t m, const uint32_t* t, const uint32_t* s, const int32_t* w);
 
+// Lets `kernel`, which has `fixed` bytes of static shared memory, be launched
+// with as much dynamic shared memory as a block can have.  The limit belongs to
+// the kernel on the device, so every context sets the same value: one that set
+// its own launch's size would, from another host thread, lower it between
+// another context's setting and its launch, which is then refused.
+template <typename... KArgs>
+void allow_shared_memory(const Ctx& c, void (*kernel)(KArgs...), size_t fixed = 0) {
+    RL_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem_optin - (int)fixed));
+}
+
 // fp32.cu (precision form)
 bool is_fp32(const Ctx& c);
 void alloc_fp32(Ctx& c);
