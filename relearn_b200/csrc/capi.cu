@@ -455,12 +455,12 @@ void plasticity_update(Ctx& c, uint32_t step) {
         }
         if (first < 3) {
             RL_CUDA_TRY(cudaEventSynchronize(c.commit_read));
-            raise_device_error(c, "synapse deletion");
             for (int t = 0; t < 3; ++t) {
                 c.stats.bound_to_delete += h[4 + t];
                 c.stats.synapses_deleted += h[7 + t];
                 note_deleted(c, h[7 + t]);
             }
+            raise_device_error(c, "synapse deletion");  // an error of any of the passes: none clears the word
         }
         c.deleted_last = first < 3;
     }

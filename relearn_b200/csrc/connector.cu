@@ -699,10 +699,6 @@ uint64_t aggregate_edges(Ctx& c, bool count_only) {
 void queue_deletion(Ctx& c, uint32_t step, int type, unsigned long long* deleted) {
     Graph& G = c.graph;
     cudaStream_t st = c.stream;
-    if (G.num_edges == 0) {
-        // nothing to delete: the elements say otherwise only if the state was set inconsistently
-        RL_CUDA_TRY(cudaMemsetAsync(c.err.p, 0, sizeof(uint32_t), st));
-    }
     DeleteArgs A;
     A.n = c.n;
     A.type = type;
@@ -713,7 +709,7 @@ void queue_deletion(Ctx& c, uint32_t step, int type, unsigned long long* deleted
     A.signal = c.nr.signal.p;
     A.enabled = c.nr.enabled.p;
     A.in_off = G.offsets.p;
-    A.out_off = G.num_edges ? G.out_off.p : G.offsets.p;  // without synapses every row is empty
+    A.out_off = G.num_edges ? G.out_off.p : G.offsets.p;  // without synapses every row is empty, and bound elements are an error
     A.out_perm = G.out_perm.p;
     A.etgt = G.tgt.p;
     A.esrc = G.src.p;
