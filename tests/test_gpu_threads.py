@@ -55,7 +55,7 @@ def test_searches_of_shallow_and_deep_octrees(precision):
         for _ in range(times):
             assert np.array_equal(net.find_targets(3), ref)
 
-    failed = together(*(lambda net=net, ref=ref, times=times: loop(net, ref, times) for net, ref, times in zip(nets, first, (1500, 1500, 700))))
+    failed = together(*(lambda net=net, ref=ref, times=times: loop(net, ref, times) for net, ref, times in zip(nets, first, (12000, 12000, 3000))))
     assert not failed, failed[:3]
     assert all(len(r) for r in first)
     for net in nets:
@@ -77,12 +77,12 @@ def test_blocks_of_small_and_large_networks(precision):
     before = [net.stats()["gpu_launches"] for net in nets]
 
     def loop(net):
-        for k in range(2000):
+        for k in range(6000):
             net.activity_block(3 + 2 * k, 2)
         net.synchronize()
 
     failed = together(*(lambda net=net: loop(net) for net in nets))
     assert not failed, failed[:3]
-    assert [net.stats()["gpu_launches"] - b for net, b in zip(nets, before)] == [4000, 4000]
+    assert [net.stats()["gpu_launches"] - b for net, b in zip(nets, before)] == [12000, 12000]
     for net in nets:
         net.close()
