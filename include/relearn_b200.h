@@ -392,6 +392,13 @@ RL_API rl_status rl_set_graphs(void* ctx, int enable);
  * counterpart in the reference (its CPU loops run step by step). */
 RL_API rl_status rl_set_step_fusion(void* ctx, int enable);
 
+/* Polls after which a thread block that waits for the others between two steps
+ * of a launch gives up (0: the default of 4,194,304, some seconds).  Such a
+ * launch returns without the block's state: the next call that has waited for
+ * it, whichever it is, and every call after that return RL_ERR_TIMEOUT, and the
+ * context can only be destroyed.  No counterpart in the reference. */
+RL_API rl_status rl_set_wait_limit(void* ctx, uint32_t polls);
+
 /* Turn per-phase CUDA-event timing on (1) or off (0). */
 RL_API rl_status rl_set_profiling(void* ctx, int enable);
 

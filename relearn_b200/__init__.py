@@ -168,7 +168,7 @@ ABI_FUNCTIONS = [
     "rl_update_connectivity", "rl_connect", "rl_process_requests", "rl_process_responses", "rl_set_elements", "rl_get_elements", "rl_set_neurons", "rl_get_neurons", "rl_set_enabled",
     "rl_add_edges", "rl_get_edges", "rl_activity_block", "rl_plasticity_update", "rl_simulate", "rl_synchronize",
     "rl_get_stats", "rl_set_stream", "rl_set_profiling", "rl_get_phase_times", "rl_prepare_update_connectivity_noalloc",
-    "rl_candidate_weights", "rl_set_graphs", "rl_set_step_fusion", "rl_ctx_memory", "rl_serve_footprint", "rl_serve_create", "rl_serve_submit", "rl_serve_poll",
+    "rl_candidate_weights", "rl_set_graphs", "rl_set_step_fusion", "rl_set_wait_limit", "rl_ctx_memory", "rl_serve_footprint", "rl_serve_create", "rl_serve_submit", "rl_serve_poll",
     "rl_serve_fetch", "rl_serve_load", "rl_serve_destroy", "rl_autotune", "rl_get_tuning", "rl_set_tuning",
     "rl_set_target_calcium", "rl_get_target_calcium", "rl_snapshot_neurons", "rl_snapshot_wait",
 ]
@@ -252,6 +252,8 @@ def load_library(path: str = LIB_PATH):
     L.rl_set_graphs.argtypes = [vp, C.c_int]
     L.rl_set_step_fusion.restype = st
     L.rl_set_step_fusion.argtypes = [vp, C.c_int]
+    L.rl_set_wait_limit.restype = st
+    L.rl_set_wait_limit.argtypes = [vp, u32]
     L.rl_connect.restype = st
     L.rl_connect.argtypes = [vp, u32, vp, u64, vp, P(u64)]
     L.rl_process_requests.restype = st
@@ -596,6 +598,11 @@ class Network:
         with synapses whose neurons all have a resident thread, in one launch
         (the default), or one launch per step; the same bits."""
         self._check(self.lib.rl_set_step_fusion(self.h, int(on)))
+
+    def set_wait_limit(self, polls: int = 0):
+        """Polls after which a wait between two steps of a launch gives up (0:
+        some seconds); the context then refuses every call (RL_ERR_TIMEOUT)."""
+        self._check(self.lib.rl_set_wait_limit(self.h, int(polls)))
 
     def set_profiling(self, on: bool = True):
         self._check(self.lib.rl_set_profiling(self.h, int(on)))

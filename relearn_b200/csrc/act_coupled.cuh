@@ -30,12 +30,18 @@ namespace rl {
 constexpr int kCoupledBlock = 384;          // threads (neurons) per block, two blocks per SM
 constexpr unsigned kCoupledCluster = 16;    // blocks per cluster (8 are portable)
 constexpr uint32_t kCoupledChunk = 16;      // steps between two replays of calcium and growth (bits of a uint16_t)
-constexpr uint32_t kCoupledPolls = 1u << 22;  // polls of a barrier before it gives up: some seconds
+
+// The barrier between the steps of a launch that counts arrivals.
+struct StepBarrier {
+    uint32_t* count;  // arrivals, in device memory
+    uint32_t* lost;   // the context's word in pinned host memory, set when a wait gives up
+    uint32_t polls;   // after so many polls
+};
 
 #if defined(__CUDACC__)
 // This block's pushes of the step are issued by all its threads.
 template <bool CLUSTER>
-__device__ __forceinline__ void step_arrive(uint32_t* count) {
+__device__ __forceinline__ void step_arrive(const StepBarrier& bar) {
     if constexpr (CLUSTER) {
         asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     } else {
@@ -43,15 +49,16 @@ __device__ __forceinline__ void step_arrive(uint32_t* count) {
         if (threadIdx.x == 0) {
             // a release at device scope, which covers what the block's other
             // threads wrote before the barrier above
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar.count) : "memory");
         }
     }
 }
 
 // Waits until `arrivals` arrivals are counted; false (in every thread of the
-// block) if the bounded wait ran out, which is recorded in *err.
+// block) if the bounded wait ran out, which the host reads in *bar.lost: the
+// blocks that gave up have not written their state, so it is no state any more.
 template <bool CLUSTER>
-__device__ __forceinline__ bool step_wait(const uint32_t* count, uint32_t arrivals, uint32_t* err) {
+__device__ __forceinline__ bool step_wait(const StepBarrier& bar, uint32_t arrivals) {
     if constexpr (CLUSTER) {
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         return true;
@@ -60,10 +67,10 @@ __device__ __forceinline__ bool step_wait(const uint32_t* count, uint32_t arriva
         if (threadIdx.x == 0) {
             uint32_t polls = 0, seen = 0;
             do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-            } while ((int32_t)(seen - arrivals) < 0 && ++polls < kCoupledPolls);
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar.count) : "memory");
+            } while ((int32_t)(seen - arrivals) < 0 && ++polls < bar.polls);
             if ((int32_t)(seen - arrivals) < 0) {
-                atomicOr(err, (uint32_t)DERR_TIMEOUT);
+                *(volatile uint32_t*)bar.lost = 1u;
                 late = 1;
             }
         }
@@ -146,6 +153,10 @@ __device__ __forceinline__ void queue_slots(bool take, uint32_t slot, uint16_t* 
 }
 #endif
 
+inline StepBarrier step_barrier(const Ctx& c) {
+    return StepBarrier{ c.act_bar.p, c.lost_word(), c.wait_polls };
+}
+
 // Launches the coupled kernel of `steps` steps (its cluster form for few blocks) if all its
 // thread blocks can be resident together; false if not.
 template <typename... KArgs, typename... Args>
@@ -193,7 +204,7 @@ bool launch_coupled(Ctx& c, uint32_t steps, void (*cluster_kernel)(KArgs...), vo
 // thread, their x, u and draws in shared memory (`bytes` per neuron), at most
 // `per_sm_target` blocks per SM; false where they do not all fit.
 template <typename Args>
-bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, uint32_t*, uint32_t*),
+bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, StepBarrier),
                            unsigned per_sm_target, size_t bytes, const Args& args, uint8_t* fired_before_last) {
     const unsigned slots = per_sm_target * (unsigned)c.num_sms;
     const uint32_t rounds = blocks_for(c.n, slots * kCoupledBlock);
@@ -220,7 +231,7 @@ bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const Ac
     cfg.attrs = at;
     cfg.numAttrs = 1;
     PhaseScope ps(c, PH_ACTIVITY_KERNEL, steps);
-    if (cudaLaunchKernelEx(&cfg, kernel, args, (const ActDesc*)c.act_desc.p, steps, rounds, fired_before_last, c.act_bar.p, c.err.p) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, kernel, args, (const ActDesc*)c.act_desc.p, steps, rounds, fired_before_last, step_barrier(c)) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }

@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(BLOCK, (MULTI ? 640 : 768) / BLOCK) k_activity
 // L1, ten dependent substeps, push, barrier), not by a pipe.
 template <int BLOCK, int H, int MODEL, bool TOP, bool CLUSTER>
 __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled(ActArgs A, const ActDesc* __restrict__ D, uint32_t nsteps,
-                                                                         uint8_t* __restrict__ fired_before_last, uint32_t* bar, uint32_t* err) {
+                                                                         uint8_t* __restrict__ fired_before_last, StepBarrier bar) {
     __shared__ double s_z[kDrawChunk * BLOCK];
     __shared__ uint16_t s_who[kDrawChunk * BLOCK];
     __shared__ uint32_t s_cnt[2];
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled(ActArgs
             if (k == 0) {
                 isum = on ? synaptic_sum(A, D, i) : 0;
             } else {
-                if (!step_wait<CLUSTER>(bar, k * gridDim.x, err)) {
+                if (!step_wait<CLUSTER>(bar, k * gridDim.x)) {
                     return;
                 }
                 if (in) {
@@ -925,7 +925,7 @@ constexpr size_t kRounds64Bytes = 3 * sizeof(double) + 2 * sizeof(uint16_t) + 1;
 template <int BLOCK, int H, int MODEL, bool TOP>
 __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled_rounds(ActArgs A, const ActDesc* __restrict__ D, uint32_t nsteps,
                                                                                 uint32_t rounds, uint8_t* __restrict__ fired_before_last,
-                                                                                uint32_t* bar, uint32_t* err) {
+                                                                                StepBarrier bar) {
     extern __shared__ double s_dyn64[];
     __shared__ uint32_t s_cnt[2];  // queued tail draws, queued spikes
     const uint32_t per = rounds * BLOCK;
@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_activity_coupled_rounds(
     for (uint32_t k = 0; k < nsteps; ++k) {
         const uint32_t step = step0 + k;
         const bool last = k + 1 == nsteps;
-        if (k > 0 && !step_wait<false>(bar, k * gridDim.x, err)) {
+        if (k > 0 && !step_wait<false>(bar, k * gridDim.x)) {
             return;
         }
         long long* in = A.syn_in[step & 1u];
@@ -1399,7 +1399,7 @@ void launch_calcium_growth64(Ctx& c, uint32_t row0, uint32_t m, cudaStream_t st)
 template <int H, int MODEL, bool TOP = false>
 bool launch_coupled64_m(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fired_before_last) {
     return launch_coupled(c, nsteps, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, true>, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, false>, A,
-                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p) ||
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, step_barrier(c)) ||
            launch_coupled_rounds(c, nsteps, &k_activity_coupled_rounds<kCoupledBlock, H, MODEL, TOP>, 768 / kCoupledBlock, kRounds64Bytes, A,
                                  fired_before_last);
 }

@@ -114,6 +114,12 @@ void raise_device_error(Ctx& c, const char* phase) {
     throw Error{ st, msg };
 }
 
+void raise_lost(const Ctx& c) {
+    if (c.h_commit != nullptr && *(volatile const uint32_t*)c.lost_word() != 0u) {
+        throw Error{ RL_ERR_TIMEOUT, "activity block: a wait at the barrier between steps ran out; the context's state is lost" };
+    }
+}
+
 namespace {
 
 template <typename T>
@@ -374,6 +380,7 @@ void create(Ctx& c, const rl_config& k, const rl_network* nets = nullptr, uint32
     RL_CUDA_TRY(cudaMemsetAsync(c.err.p, 0, sizeof(uint32_t), c.stream));
     c.commit_cnt.alloc(kCommitCounts);
     c.h_commit = pinned_slot_take();
+    *(volatile uint32_t*)c.lost_word() = 0u;
     RL_CUDA_TRY(cudaEventCreateWithFlags(&c.commit_read, cudaEventDisableTiming));
     c.counters.alloc(4);
     RL_CUDA_TRY(cudaMemsetAsync(c.counters.p, 0, 4 * sizeof(uint64_t), c.stream));
@@ -427,6 +434,7 @@ void plasticity_update(Ctx& c, uint32_t step) {
             update_tree(c);
         }
         RL_CUDA_TRY(cudaStreamSynchronize(c.stream));
+        raise_lost(c);
         const unsigned long long* h = c.h_commit;
         c.stats.bound_to_delete += h[0] + h[1] + h[2];
         const int first = h[0] ? 0 : (h[1] ? 1 : (h[2] ? 2 : 3));
@@ -562,7 +570,9 @@ rl_status guarded(void* ctx, F&& f) {
     Bind bind(c);
     try {
         RL_CUDA_TRY(cudaSetDevice(c.device));
+        raise_lost(c);
         f(c);
+        raise_lost(c);  // what the call read, it read behind the launch that gave up
         return RL_OK;
     } catch (const Error& e) {
         c.last_error = e.message;
@@ -1290,6 +1300,10 @@ rl_status rl_internal_set_fused_work(void* ctx, uint64_t work) {
 
 rl_status rl_set_step_fusion(void* ctx, int enable) {
     return rl::guarded(ctx, [&](Ctx& c) { c.step_fusion = enable != 0; });
+}
+
+rl_status rl_set_wait_limit(void* ctx, uint32_t polls) {
+    return rl::guarded(ctx, [&](Ctx& c) { c.wait_polls = polls ? polls : rl::kWaitPolls; });
 }
 
 rl_status rl_set_profiling(void* ctx, int enable) {

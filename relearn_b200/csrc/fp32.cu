@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(BLOCK) k_activity_f32_steps(Act32 A, const Act
 // so the bits are theirs.
 template <int BLOCK, int H, int MODEL, bool CLUSTER>
 __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled(Act32 A, const ActDesc* __restrict__ D, uint32_t nsteps,
-                                                                             uint8_t* __restrict__ fired_before_last, uint32_t* bar, uint32_t* err) {
+                                                                             uint8_t* __restrict__ fired_before_last, StepBarrier bar) {
     const uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
     const bool in = i < A.n;
     const bool en = in && A.enabled[i] != 0;
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled(Ac
         }
         int pushed = 0;
         if (k > 0) {
-            if (!step_wait<CLUSTER>(bar, k * gridDim.x, err)) {
+            if (!step_wait<CLUSTER>(bar, k * gridDim.x)) {
                 return;
             }
             if (in) {
@@ -705,7 +705,7 @@ constexpr size_t kRounds32Bytes = 3 * sizeof(float) + 2 * sizeof(uint16_t) + 1;
 template <int BLOCK, int H, int MODEL>
 __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled_rounds(Act32 A, const ActDesc* __restrict__ D, uint32_t nsteps,
                                                                                     uint32_t rounds, uint8_t* __restrict__ fired_before_last,
-                                                                                    uint32_t* bar, uint32_t* err) {
+                                                                                    StepBarrier bar) {
     extern __shared__ float s_dyn32[];
     __shared__ uint32_t s_cnt;  // queued spikes
     const uint32_t per = rounds * BLOCK;
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_activity_f32_coupled_ro
     for (uint32_t k = 0; k < nsteps; ++k) {
         const uint32_t step = step0 + k;
         const bool last = k + 1 == nsteps;
-        if (k > 0 && !step_wait<false>(bar, k * gridDim.x, err)) {
+        if (k > 0 && !step_wait<false>(bar, k * gridDim.x)) {
             return;
         }
         int32_t* in = A.syn_in[step & 1u];
@@ -2131,7 +2131,7 @@ namespace {
 template <int H, int MODEL>
 bool launch_coupled32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_before_last) {
     return launch_coupled(c, nsteps, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, true>, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, false>, A,
-                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, c.act_bar.p, c.err.p) ||
+                          (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, step_barrier(c)) ||
            launch_coupled_rounds(c, nsteps, &k_activity_f32_coupled_rounds<kCoupledBlock, H, MODEL>, 1152 / kCoupledBlock, kRounds32Bytes, A,
                                  fired_before_last);
 }

@@ -67,6 +67,7 @@ extern "C" RL_API rl_status rl_prepare_update_connectivity_noalloc(void* ctx, co
     } restore{ prev_device };
     const rl::Binding prev_bind = rl::g_bind;
     try {
+        rl::raise_lost(c);
         RL_CHECK(c.positions_set, RL_ERR_INVALID, "rl_set_positions has not been called");
         RL_CHECK(d_vacant_exc && d_vacant_inh, RL_ERR_INVALID, "device vacancy arrays are required");
         RL_CHECK(c.tree.num_nodes <= kMaxNodes, RL_ERR_OVERFLOW,

@@ -259,7 +259,8 @@ struct KernelParams {
 // Counts of an update (Ctx::commit_cnt), and the pinned words behind their host copy.
 constexpr size_t kCommitCounts = 10;
 constexpr size_t kReadSlot = 12;
-constexpr int kReadError = 0, kReadA = 1, kReadB = 2;
+constexpr int kReadError = 0, kReadA = 1, kReadB = 2, kReadLost = 3;
+constexpr uint32_t kWaitPolls = 1u << 22;  // polls of a wait in a kernel before it gives up: some seconds
 
 struct Ctx;
 // Records an event pair around a scope when profiling is on.
@@ -391,6 +392,8 @@ struct Ctx {
     DBuf<unsigned long long> commit_cnt;
     unsigned long long* h_commit = nullptr;  // pinned host copy of commit_cnt (read without blocking the enqueue), then the words of read_slot
     uint32_t* read_slot() const;             // pinned words for small reads (kRead*)
+    uint32_t* lost_word() const { return read_slot() + kReadLost; }  // set by a launch whose wait gave up (raise_lost)
+    uint32_t wait_polls = kWaitPolls;
     cudaEvent_t commit_read = nullptr;       // the counts of an update's deletions have landed
     bool target_uniform = true;  // every neuron has cfg.target_calcium as its target
     // Host transfers that overlap the work on the context's stream: uploads
@@ -544,5 +547,9 @@ void launch_commit_f32(Ctx& c, int type, unsigned long long* total, const unsign
 void check_device_error(Ctx& c, const char* phase);
 void queue_error_read(Ctx& c);                        // the same in two parts: copy the error word ...
 void raise_device_error(Ctx& c, const char* phase);   // ... and, after a synchronisation, throw if it is set
+// Throws if a launch that has completed gave up at the barrier between its
+// steps.  Such a launch leaves the context without a state: every entry point
+// asks before it starts and when it is done, and none clears it.
+void raise_lost(const Ctx& c);
 
 }  // namespace rl
