@@ -202,10 +202,11 @@ bool launch_coupled(Ctx& c, uint32_t steps, void (*cluster_kernel)(KArgs...), vo
 
 // The form for more neurons than resident threads: `rounds` neurons per
 // thread, their x, u and draws in shared memory (`bytes` per neuron), at most
-// `per_sm_target` blocks per SM; false where they do not all fit.
-template <typename Args>
-bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, StepBarrier),
-                           unsigned per_sm_target, size_t bytes, const Args& args, uint8_t* fired_before_last) {
+// `per_sm_target` blocks per SM; false where they do not all fit.  `bar` is the
+// barrier as the kernel takes it.
+template <typename Args, typename... Bar>
+bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, Bar...), unsigned per_sm_target,
+                           size_t bytes, const Args& args, uint8_t* fired_before_last, Bar... bar) {
     const unsigned slots = per_sm_target * (unsigned)c.num_sms;
     const uint32_t rounds = blocks_for(c.n, slots * kCoupledBlock);
     const unsigned blocks = blocks_for(c.n, rounds * kCoupledBlock);
@@ -231,7 +232,7 @@ bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const Ac
     cfg.attrs = at;
     cfg.numAttrs = 1;
     PhaseScope ps(c, PH_ACTIVITY_KERNEL, steps);
-    if (cudaLaunchKernelEx(&cfg, kernel, args, (const ActDesc*)c.act_desc.p, steps, rounds, fired_before_last, step_barrier(c)) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, kernel, args, (const ActDesc*)c.act_desc.p, steps, rounds, fired_before_last, bar...) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }

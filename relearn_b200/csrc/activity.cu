@@ -1401,7 +1401,7 @@ bool launch_coupled64_m(Ctx& c, const ActArgs& A, uint32_t nsteps, uint8_t* fire
     return launch_coupled(c, nsteps, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, true>, &k_activity_coupled<kCoupledBlock, H, MODEL, TOP, false>, A,
                           (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, step_barrier(c)) ||
            launch_coupled_rounds(c, nsteps, &k_activity_coupled_rounds<kCoupledBlock, H, MODEL, TOP>, 768 / kCoupledBlock, kRounds64Bytes, A,
-                                 fired_before_last);
+                                 fired_before_last, step_barrier(c));
 }
 
 template <int H>
