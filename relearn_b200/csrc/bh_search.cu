@@ -448,9 +448,6 @@ __device__ __forceinline__ void search_task(const SearchArgs& A, const Hot64& H,
     if (active) {
         A.target[idx] = result;
     }
-    if (A.redo_only) {
-        return;  // counted by the form that left them
-    }
     // touched-node counter (reference-equivalent acceptance tests)
     unsigned long long t = touched;
     for (int o = 16; o > 0; o >>= 1) {
@@ -596,6 +593,16 @@ __device__ int32_t wide_search(const SearchArgs& S, uint32_t cap, const WideSlot
     return -1;
 }
 
+// Adds the warp's acceptance tests to the touched-node counter.
+__device__ __forceinline__ void add_touched(unsigned long long* counter, unsigned long long touched) {
+    for (int o = 16; o > 0; o >>= 1) {
+        touched += __shfl_down_sync(0xFFFFFFFFu, touched, o);
+    }
+    if ((threadIdx.x & 31u) == 0u) {
+        atomicAdd(counter, touched);
+    }
+}
+
 // Persistent warps, one search per task.
 template <int WPB>
 __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide(WideArgs A) {
@@ -626,8 +633,9 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide(WideArgs A) {
         const uint32_t seg = wide_entry_segment(idx, S.seg_begin, S.num_segs);
         const NetInfo& N = S.nets[S.seg_net[seg]];
         const WarpNet W{ N.theta, N.scale, N.seed, S.seg_net[seg], N.first };
-        uint32_t again = 0;  // the bins form has counted this search's acceptance tests
-        const int32_t result = wide_search(S, A.cap, P, W, S.list_src[idx], S.list_j[idx], s_round, again);
+        uint32_t tests = 0;
+        const int32_t result = wide_search(S, A.cap, P, W, S.list_src[idx], S.list_j[idx], s_round, tests);
+        touched += result != kRedo ? tests : 0u;  // else counted by the packets
         if (lane == 0) {
             S.target[idx] = result;
             if (result == kRedo) {
@@ -636,6 +644,7 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_search_wide(WideArgs A) {
         }
         __syncwarp();
     }
+    add_touched(A.touched, touched);
 }
 
 // ------------------------------------------------- one search per warp, by bins
@@ -782,16 +791,18 @@ __global__ void __launch_bounds__(WPB * 32, SQUARED ? 24 / WPB : 16 / WPB) k_sea
         const NetInfo& N = S.nets[S.seg_net[lo]];
         const WarpNet W{ N.theta, N.scale, N.seed, S.seg_net[lo], N.first };
         int32_t result = -1;
+        uint32_t tests = 0;
         if (!N.root_leaf) {
             const uint32_t source = S.list_src[idx];
             const uint32_t j = S.list_j[idx];
             const Bins64<SQUARED> ev{ S, W, S.rec, S.meta, tab, S.px[source], S.py[source], S.pz[source], W.scale, W.scale * 92.332482616893656768,
                                       (float)(W.theta * W.theta),
                                       (float)fmin(-699.0 / W.scale, 3e38), source, S.num_nodes };
-            result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny64, touched, ev,
+            result = bins_search(M, S.meta, A.parent, S.num_nodes, W.root, __ldg(&S.leaf_of[source]), kBinsTiny64, tests, ev,
                                  [&](double total, uint32_t depth) { return pick_threshold(total, W.seed, S.step, source - W.first, j, depth); },
                                  [&](double total, uint32_t visited) { return total * (kBinsMargin64 + (double)visited * 4.5e-16); });
         }
+        touched += result != kRedo ? tests : 0u;  // else counted by the form that finishes the search
         if (lane == 0) {
             S.target[idx] = result;
             if (result == kRedo) {
@@ -800,13 +811,7 @@ __global__ void __launch_bounds__(WPB * 32, SQUARED ? 24 / WPB : 16 / WPB) k_sea
         }
         __syncwarp();
     }
-    unsigned long long sum = touched;
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
-    }
-    if (lane == 0) {
-        atomicAdd(A.touched, sum);
-    }
+    add_touched(A.touched, touched);
 }
 
 using SearchKernel = void (*)(SearchArgs);
