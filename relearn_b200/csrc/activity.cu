@@ -108,7 +108,8 @@ __device__ __forceinline__ double growth_curve_pre(double current, double eta, i
 
 // growth_curve_pre without branches (the eta == epsilon case selected), for
 // the software-pipelined block kernel.  Equality with eta is compared on the
-// bits (a calcium after its step is never -0, and NaN equals nothing).
+// bits (a calcium after its step is never -0 for tau_c > 0, act64_args makes eta
+// +0 if it is -0, and NaN equals nothing).
 __device__ __forceinline__ double growth_curve_flat(double current, double eta, int flat, double xi, double zeta, double zeta_inv) {
     const double diff = current - xi;
     const double q0 = diff * zeta_inv;
@@ -1292,7 +1293,7 @@ ActArgs act64_args(Ctx& c, uint32_t kstep, const uint8_t* fired_prev, uint8_t* f
     A.tau_inv = -1.0 / k.tau_c;
     A.scale_c = 1.0 / (double)k.h_calcium;
     for (int t = 0; t < 3; ++t) {
-        A.eta[t] = k.min_calcium[t];
+        A.eta[t] = k.min_calcium[t] + 0.0;  // -0 becomes +0, for growth_curve_flat
     }
     A.nets = c.d_nets.p;
     A.net_of = c.net_of.p;
