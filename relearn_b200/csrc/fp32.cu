@@ -1735,12 +1735,7 @@ struct BinsArgs32 {
     uint32_t* counts;  // per type: entries of redo
 };
 
-// The Kahan sums of n FP32 weights lie within (2 + n 2^-24) 2^-24 of the exact
-// ones, r within 3 x 2^-24 of the exact total's share (its total and one
-// rounding), and the bins' FP64 sums within n 2^-53: 5.1 x 2^-24 of the total
-// together for any n that fits an octree.  Totals below kBinsTiny32 (weights
-// in the subnormal range) are left to the ordered form.
-constexpr double kBinsMargin32 = 3.3e-7;
+// Totals below this (weights in the subnormal range) are left to the ordered form.
 constexpr double kBinsTiny32 = 1e-30;
 
 // eval32's operations without its branches (the Gaussian kernel): the same
@@ -1833,7 +1828,7 @@ __global__ void __launch_bounds__(WPB * 32, 20 / WPB) k_search_bins32(BinsArgs32
                                      const double r = (double)(w.x >> 8) * 5.9604644775390625e-8 * total;
                                      return r > 0.0 ? r : 1.0e-38;
                                  },
-                                 [&](double total, uint32_t) { return total * kBinsMargin32; });
+                                 [&](double total, uint32_t visited) { return bins_margin32(total, visited); });
         }
         if (lane == 0) {
             S.target[idx] = result;

@@ -688,6 +688,17 @@ RL_HD double uniform_from_bits53(uint64_t b) {
     return base - (high ? 0.0 : as_f64(0x3FDFFFFFFFFFFFFFull));
 }
 
+// FP32 search by bins: bound on the difference between its running sums (and
+// its r) and the ordered form's, for a total of `visited` nodes.  With
+// u = 2^-24, a Kahan sum of n positive weights lies within 2 u + O(n u^2) of
+// the exact one (Goldberg, "What every computer scientist should know about
+// floating-point arithmetic", ACM Comput. Surv. 23 (1991), theorem 8; 8 n u^2
+// covers the second term), r within one u more of the exact total's share, and
+// the bins' FP64 sums within n 2^-53 each: 5 u + 16 n u^2 + n 2^-52.
+RL_HD double bins_margin32(double total, uint32_t visited) {
+    return total * (3.0e-7 + (double)visited * 5.8e-14);
+}
+
 // The open-interval uniform of a neuron's background draw.
 RL_HD double noise_uniform(uint64_t seed, uint32_t step, uint32_t neuron) {
     const u32x4 r = noise_block(seed, step, neuron);
