@@ -393,7 +393,8 @@ RL_API rl_status rl_set_graphs(void* ctx, int enable);
 RL_API rl_status rl_set_step_fusion(void* ctx, int enable);
 
 /* Polls after which a thread block that waits for the others between two steps
- * of a launch gives up (0: the default of 4,194,304, some seconds).  Such a
+ * of a launch gives up (0: the default of 4,194,304, some seconds; one more per
+ * two synapses of the network, which a single neuron may hold).  Such a
  * launch returns without the block's state: the next call that has waited for
  * it, whichever it is, and every call after that return RL_ERR_TIMEOUT, and the
  * context can only be destroyed.  No counterpart in the reference. */

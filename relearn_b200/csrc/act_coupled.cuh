@@ -23,6 +23,8 @@
 // 21.2 -> 19.0, 1M 38.0 -> 33.7; FP32 7.1 -> 5.2, 12.6 -> 8.5, 21.5 -> 14.4).
 #pragma once
 
+#include <algorithm>
+
 #include "rl_context.cuh"
 
 namespace rl {
@@ -153,8 +155,15 @@ __device__ __forceinline__ void queue_slots(bool take, uint32_t slot, uint16_t* 
 }
 #endif
 
+// The polls of a wait: one neuron may hold every synapse, and its block then
+// walks the list alone while the others wait (up to 75 ns per synapse; a poll
+// takes about 700).
+inline uint32_t barrier_polls(const Ctx& c) {
+    return (uint32_t)std::min<uint64_t>(0xFFFFFFFFull, c.wait_polls + c.graph.num_edges / 2u);
+}
+
 inline StepBarrier step_barrier(const Ctx& c) {
-    return StepBarrier{ c.act_bar.p, c.lost_word(), c.wait_polls };
+    return StepBarrier{ c.act_bar.p, c.lost_word(), barrier_polls(c) };
 }
 
 // Launches the coupled kernel of `steps` steps (its cluster form for few blocks) if all its

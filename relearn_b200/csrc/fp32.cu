@@ -2132,7 +2132,7 @@ bool launch_coupled32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_be
     return launch_coupled(c, nsteps, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, true>, &k_activity_f32_coupled<kCoupledBlock, H, MODEL, false>, A,
                           (const ActDesc*)c.act_desc.p, nsteps, fired_before_last, step_barrier(c)) ||
            launch_coupled_rounds(c, nsteps, &k_activity_f32_coupled_rounds<kCoupledBlock, H, MODEL>, 1152 / kCoupledBlock, kRounds32Bytes, A,
-                                 fired_before_last, c.act_bar.p, c.lost_word(), c.wait_polls);
+                                 fired_before_last, c.act_bar.p, c.lost_word(), barrier_polls(c));
 }
 
 }  // namespace

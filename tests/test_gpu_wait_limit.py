@@ -14,13 +14,13 @@ RL_ERR_TIMEOUT = 4
 SIZES = [20_011, 180_001]
 
 
-def network(n, precision):
+def network(n, precision, edges=1):
     params, pos, sig = small_network(n, 2500.0, 11)
     params["precision"] = precision
     net = R.Network(params)
     net.set_positions(pos, sig)
     rng = np.random.default_rng(n)
-    net.add_edges(rng.integers(0, n, 4 * n), rng.integers(0, n, 4 * n), np.ones(4 * n, np.int32))
+    net.add_edges(rng.integers(0, n, edges), rng.integers(0, n, edges), np.ones(edges, np.int32))
     return net
 
 
@@ -58,10 +58,10 @@ def test_lost_block_is_reported_and_stays_refused(read, n, precision):
 
 @pytest.mark.parametrize("precision", [0, 1])
 def test_other_contexts_go_on(precision):
-    ref = network(SIZES[0], precision)
+    ref = network(SIZES[0], precision, 80_000)
     ref.set_step_fusion(False)
     ref.activity_block(1, 100)
-    net = network(SIZES[0], precision)
+    net = network(SIZES[0], precision, 80_000)
     lost = network(SIZES[1], precision)
     lost.set_wait_limit(1)
     lost.activity_block(1, 50)
@@ -77,3 +77,21 @@ def test_other_contexts_go_on(precision):
     again.synchronize()
     for net in (ref, net, again):
         net.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("hub", ["target", "source"])
+def test_limit_leaves_room_for_a_neuron_with_every_synapse(hub, n, precision):
+    """Its block walks the whole list by itself, tens of milliseconds, while
+    the others wait; the limit set here is well below one."""
+    net = network(n, precision)
+    m = 600_000
+    one, many = np.zeros(m, np.uint32), np.random.default_rng(2).integers(0, n, m).astype(np.uint32)
+    net.add_edges(one if hub == "target" else many, one if hub == "source" else many, np.ones(m, np.int32))
+    net.set_neurons(fired=np.ones(n, np.uint8))
+    net.set_enabled((np.arange(n) > 0).astype(np.uint8) if hub == "source" else np.ones(n, np.uint8))  # keeps its spike flag
+    net.set_wait_limit(100)
+    net.activity_block(1, 4)
+    net.synchronize()
+    net.close()
