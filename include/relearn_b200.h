@@ -422,7 +422,8 @@ typedef struct rl_tuning {
     int32_t search_warps;    /* 2, 4 or 8 */
     int32_t search_hot;      /* 0, or 1024 / 4096 top octree nodes in shared memory (search_warps 32) */
     int32_t search_packet;   /* 32, 16, 4 or 1 searches of Morton-adjacent sources walking the first descent together;
-                                0: one search per warp (search_warps 4), the shape without tuning */
+                                0: one search per warp (search_warps 4).  Without tuning the library takes 0, or 32
+                                (search_warps 2, search_cap 1) for dense lists where that is faster */
     int32_t search_cap;      /* 1: registers capped at 64 (more resident warps), 0: as compiled */
     int32_t act_block;       /* 128, 256 or 512 */
     int32_t act_persistent;  /* 0 or 1 */

@@ -1058,9 +1058,36 @@ void launch_wide(Ctx& c, const SearchArgs (&a)[2], const uint32_t (&warps)[2]) {
 
 }  // namespace
 
-// Whether the tuner times a candidate shape on this context's search list.
-bool search_variant_applies(const Ctx&, const SearchVariant&) {
-    return true;
+// The shape for a list of m searches without tuning: one search per warp by
+// bins, except for lists so dense that a packet's 32 sources walk the same way,
+// and so long that packets fill the device, where the bins form has no shorter
+// evaluation to offer (packets -> bins, ms; every neuron searching):
+//   * FP64 without the squared evaluation: gamma kernel 500,000 neurons 40.2 ->
+//     35.1, 700,000 51.0 -> 51.5, 2M 143 -> 163; linear kernel (300 um) 35.3 ->
+//     35.3, 45.4 -> 51.6, 128 -> 162; half of 1M neurons searching 48.3 -> 38.4;
+//   * FP32, kernels other than the Gaussian: gamma 500,000 neurons 17.8 -> 17.4,
+//     600,000 19.9 -> 21.2, 2M 64.0 -> 79.5; half of 1M 21.3 -> 19.1;
+//   * FP32 at a small theta, where the many nodes of a walk leave many picks
+//     within the margin: theta 0.1, 20,000 neurons 16.5 -> 15.9, 100,000 48.1 ->
+//     56.6; theta 0.15, 100,000 25.4 -> 23.5, 400,000 61.1 -> 65.1.
+// Elsewhere bins win: Gaussian 1M neurons FP64 71.6 -> 32.1, FP32 32.7 -> 23.6;
+// 20,000 searches among them 47 -> 0.80; 260 of 52,000 neurons 23 -> 0.11.
+SearchVariant default_search_shape(const Ctx& c, uint64_t m) {
+    const SearchVariant packets{ 2, 32, 1, 0 };
+    if (4 * m < 3 * (uint64_t)c.n) {
+        return SearchVariant{};
+    }
+    if (!is_fp32(c)) {
+        return m >= 650'000 && !bins_squared(c) ? packets : SearchVariant{};
+    }
+    if (c.kernel.type != RL_KERNEL_GAUSSIAN && m >= 550'000) {
+        return packets;
+    }
+    double theta = 0.0;
+    for (const NetInfo& N : c.nets) {
+        theta = std::max(theta, N.theta);
+    }
+    return (theta <= 0.11 && m >= 60'000) || (theta <= 0.16 && m >= 300'000) ? packets : SearchVariant{};
 }
 
 // Searches that the bins form left open go one per warp, unless a large share
@@ -1086,10 +1113,6 @@ void tune_search(Ctx& c, F&& launch_all) {
     float best = 1e30f;
     SearchVariant pick = c.tune.search;
     for (const SearchVariant& v : search_variants()) {
-        if (!search_variant_applies(c, v)) {
-            c.tune.search_ms.push_back(0.0f);  // keeps the times in candidate order
-            continue;
-        }
         launch_all(v);
         RL_CUDA_TRY(cudaEventRecord(e0, st));
         launch_all(v);
@@ -1129,8 +1152,7 @@ const std::vector<SearchVariant>& search_variants() {
                 out.push_back(SearchVariant{ 32, p, 1, hot });
             }
         }
-        // one search per warp (packet 0; FP64 form, large networks): for
-        // search lists whose sources lie far apart
+        // one search per warp (packet 0)
         out.push_back(SearchVariant{ 4, 0, 0, 0 });
         return out;
     }();
@@ -1323,6 +1345,9 @@ void run_search(Ctx& c, uint32_t step) {
                 c.tune.search_by_class[dc] = c.tune.search;
             }
             c.tune.search_state = TUNE_DONE;
+            c.tune.search_set = true;
+        } else if (!c.tune.search_set) {
+            c.tune.search = default_search_shape(c, m);
         }
         {
             PhaseScope ps(c, PH_SEARCH_KERNEL);

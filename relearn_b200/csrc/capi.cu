@@ -1377,6 +1377,7 @@ rl_status rl_set_tuning(void* ctx, const rl_tuning* t) {
         c.tune.search = rl::SearchVariant{ t->search_warps, t->search_packet, t->search_cap, t->search_hot };
         c.tune.act = rl::ActVariant{ t->act_block, t->act_persistent, t->act_vec };
         c.tune.search_state = rl::TUNE_OFF;
+        c.tune.search_set = true;
         c.tune.act_state = rl::TUNE_OFF;
         rl::drop_activity_graphs(c);
     });

@@ -291,12 +291,9 @@ struct ActDesc {
     const uint32_t* tgt;
 };
 
-// Launch shape of the Barnes-Hut search kernels.
-// Without tuning: one search per warp by bins (packet 0), the fastest form in
-// every density class measured (1M neurons, every neuron searching: 32.7 ms
-// against 72.3 ms for packets of 32 in FP64, 25.3 against 33.4 ms in FP32;
-// 20,000 searches: 0.80 against 47 ms; 52,000 neurons, 260 searches: 0.11
-// against 23 ms).
+// Launch shape of the Barnes-Hut search kernels.  Without tuning
+// default_search_shape picks between the first (one search per warp by bins)
+// and packets of 32.
 struct SearchVariant {
     int warps = 4;    // warps per block
     int packet = 0;   // lanes (sources) that walk the descent from the root together; 0: one search per warp
@@ -304,7 +301,6 @@ struct SearchVariant {
     int hot = 0;      // > 0: persistent form, one block of 32 warps per SM with up
                       // to `hot` top octree nodes in shared memory
 };
-
 
 // Launch shape of the activity kernel.
 struct ActVariant {
@@ -319,6 +315,7 @@ enum : int { TUNE_OFF = 0, TUNE_REQUESTED = 1, TUNE_DONE = 2 };
 struct Tuning {
     SearchVariant search;
     ActVariant act;
+    bool search_set = false;       // the search shape is the caller's or the tuner's
     int search_state = TUNE_OFF;
     int act_state = TUNE_OFF;
     bool force = false;            // time again even when the process has a result for this shape
@@ -329,7 +326,7 @@ struct Tuning {
 };
 
 const std::vector<SearchVariant>& search_variants();
-bool search_variant_applies(const Ctx& c, const SearchVariant& v);
+SearchVariant default_search_shape(const Ctx& c, uint64_t m);
 bool wide_redo_by_packets(const Ctx& c, uint64_t open);
 struct WideSlot;
 uint32_t wide_cap(const Ctx& c);
