@@ -1090,11 +1090,16 @@ SearchVariant default_search_shape(const Ctx& c, uint64_t m) {
     return (theta <= 0.11 && m >= 60'000) || (theta <= 0.16 && m >= 300'000) ? packets : SearchVariant{};
 }
 
-// Searches that the bins form left open go one per warp, unless a large share
-// of a dense list is open (totals that underflow): then packets of Morton
-// neighbours are faster.
+// Searches that the bins form left open go one per warp, each at its price
+// (0.17-0.30 us in FP64, 0.19-0.37 in FP32 at theta 0.3), unless they are so
+// many, and so large a share of the list, that a pass in packets over the list
+// is cheaper.  Lists whose totals underflow in the main (sigma 0.2 um; FP64 six
+// searches in ten open, FP32 all), 20,000, 100,000 and 400,000 neurons
+// searching, ordered against packets: FP64 2.1, 13.6; 14.8, 26.2; 75, 58 ms;
+// FP32 3.7, 7.5; 28, 14.4; 148, 33 ms; 120,000 of 400,000 neurons searching:
+// FP64 23, 39; FP32 45, 23 ms.
 bool wide_redo_by_packets(const Ctx& c, uint64_t open) {
-    return open > 4096 && 8 * open > c.search.num_searches && search_density_class(c.n, c.search.num_searches) == 0;
+    return open > (is_fp32(c) ? 60'000u : 250'000u) && 8 * open > c.search.num_searches;
 }
 
 // Times every search variant that fits the octree on the current search list

@@ -37,7 +37,9 @@ ROUTES = {"bins": -1, "ordered": 0, "packets": 1, "ordered, then packets": 2}
     ("underflow", 2500, dict(sigma=0.2), 1.0, "ordered"),
     ("far", 2500, dict(sigma=1.5), 1.0, ("bins", "ordered")),  # weights below FP32's range, not FP64's
     ("cutoff", 2500, dict(kernel_type=R.KERNEL_LINEAR, linear_cutoff=4.0), 1.0, "ordered"),
-    ("underflow, many", 20000, dict(sigma=0.2), 1.0, "packets"),
+    ("underflow, many", 20000, dict(sigma=0.2), 1.0, "ordered"),
+    ("underflow, more", 64000, dict(sigma=0.2), 1.0, ("ordered", "packets")),
+    ("underflow, most", 290000, dict(sigma=0.1), 1.0, "packets"),
     ("underflow, sparse", 20000, dict(sigma=0.2), 0.01, "ordered"),
     ("long walks", 20000, dict(sigma=0.2, theta=0.05), 0.02, "ordered, then packets"),
 ])
