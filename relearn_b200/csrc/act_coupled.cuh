@@ -19,8 +19,9 @@
 // and count arrivals in device memory (6,200 neurons: 3.7 and 3.1 us).
 // More neurons than resident threads run in rounds, several per thread with
 // their state in shared memory (up to 1,136,640 neurons FP64, 1,875,456 FP32;
-// untuned launch per step -> here: FP64 171,000 neurons 12.8 -> 8.8, 500,000
-// 21.2 -> 19.0, 1M 38.0 -> 33.7; FP32 7.1 -> 5.2, 12.6 -> 8.5, 21.5 -> 14.4).
+// one launch per step -> here, four synapses per neuron: FP64 300,000 neurons
+// 14.4 -> 11.8, 600,000 24.9 -> 21.2, 1M 38.6 -> 32.0 (37.9 with the shape the
+// tuner picks); FP32 9.4 -> 6.3, 14.4 -> 10.0, 21.4 -> 14.3 (tuned 19.6)).
 #pragma once
 
 #include <algorithm>
@@ -122,6 +123,34 @@ __device__ __forceinline__ void push_warp(bool f, uint32_t o0, uint32_t o1, cons
     __syncwarp();
 }
 
+// Edges j, j + 8, ... below end of the out-CSR order, four at a time, so that
+// their dependent loads lie side by side (one at a time -> four, us per step:
+// 600,000 neurons with 20 synapses each FP64 29.4 -> 25.1, FP32 18.8 -> 14.2;
+// 300,000 with 100 71.4 -> 68.8 and 67.9 -> 61.0).
+template <typename T>
+__device__ __forceinline__ void push_edges(uint32_t j, uint32_t end, const uint32_t* __restrict__ out_perm, const uint32_t* __restrict__ tgt,
+                                           const int32_t* __restrict__ w, T* next) {
+    for (; j < end; j += 32u) {
+        uint32_t e[4], t[4];
+        int32_t v[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            e[q] = j + 8u * q < end ? out_perm[j + 8u * q] : 0u;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            t[q] = j + 8u * q < end ? tgt[e[q]] : 0u;
+            v[q] = j + 8u * q < end ? w[e[q]] : 0;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            if (j + 8u * q < end) {
+                add_weight(next + t[q], v[q]);
+            }
+        }
+    }
+}
+
 // The block's queued spikes (neurons base + who[q]), eight lanes each.
 template <int BLOCK, typename T>
 __device__ __forceinline__ void push_queue(uint32_t cnt, uint32_t base, const uint16_t* who, const uint32_t* __restrict__ out_off,
@@ -129,11 +158,7 @@ __device__ __forceinline__ void push_queue(uint32_t cnt, uint32_t base, const ui
                                            T* next) {
     for (uint32_t q = threadIdx.x >> 3; q < cnt; q += BLOCK / 8) {
         const uint32_t i = base + who[q];
-        const uint32_t o1 = out_off[i + 1];
-        for (uint32_t j = out_off[i] + (threadIdx.x & 7u); j < o1; j += 8u) {
-            const uint32_t e = out_perm[j];
-            add_weight(next + tgt[e], w[e]);
-        }
+        push_edges(out_off[i] + (threadIdx.x & 7u), out_off[i + 1], out_perm, tgt, w, next);
     }
 }
 
