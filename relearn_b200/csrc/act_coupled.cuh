@@ -234,10 +234,41 @@ bool launch_coupled(Ctx& c, uint32_t steps, void (*cluster_kernel)(KArgs...), vo
     return true;
 }
 
+// Whether a block of `steps` steps in `rounds` neurons for each of `threads`
+// threads beats one launch per step (us per step, one launch per step against
+// rounds).  It does for the Izhikevich and Poisson models (above) unless
+//   * the synapse list is so long that walking it at each step's end, with
+//     nothing beside it, takes longer than the rest: FP64 30M synapses 74, 63
+//     (1M neurons) and 67.8, 68.8 (300,000), 36M 67.8, 68.9, 40M 85, 91, 60M
+//     121, 188; FP32 40M 71.6, 45.4, 50M 88.9, 80.8, 60M 102, 104 and 116, 150;
+//   * FP64 has only two steps to spread its loads and stores over: 850,000
+//     neurons 41.1, 43.0 (three steps 46.1, 38.5).
+// The other models' longer substeps leave less to gain: AEIF FP64 400,000
+// neurons (4 rounds) 26.6, 25.5, 700,000 (7) 42.4, 44.5; FitzHugh-Nagumo, of
+// whose neurons two in five fire at a step, FP64 300,000 (3) 20.1, 19.4,
+// 400,000 (4) 23.6, 24.9; FP32 where the last round is nearly full: 500,000 (3
+// rounds, 98 %) 20.7, 18.8, 700,000 (5, 82 %) 26.8, 29.0, 250,000 (2, 73 %)
+// 13.9, 13.1, 200,000 (2, 59 %) 9.8, 10.9, and the L1 cache is left some room:
+// 1.4M (9) 60.5, 59.4, 1.87M (11) 92.6, 129.
+inline bool rounds_pay(const Ctx& c, uint32_t steps, uint32_t rounds, uint64_t threads) {
+    const bool fp32 = is_fp32(c);
+    if (c.graph.num_edges > (fp32 ? 56'000'000u : 32'000'000u) || (!fp32 && steps < 3)) {
+        return false;
+    }
+    if (c.cfg.neuron_model == RL_MODEL_AEIF) {
+        return fp32 || rounds <= 4;
+    }
+    if (c.cfg.neuron_model == RL_MODEL_FITZHUGH_NAGUMO) {
+        const double used = (double)c.n / (double)(rounds * threads);
+        return fp32 ? rounds <= 9 && used >= (rounds == 2 ? 0.7 : 0.9) : rounds <= 3;
+    }
+    return true;
+}
+
 // The form for more neurons than resident threads: `rounds` neurons per
 // thread, their x, u and draws in shared memory (`bytes` per neuron), at most
-// `per_sm_target` blocks per SM; false where they do not all fit.  `bar` is the
-// barrier as the kernel takes it.
+// `per_sm_target` blocks per SM; false where they do not all fit, or would not
+// be faster.  `bar` is the barrier as the kernel takes it.
 template <typename Args, typename... Bar>
 bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const ActDesc*, uint32_t, uint32_t, uint8_t*, Bar...), unsigned per_sm_target,
                            size_t bytes, const Args& args, uint8_t* fired_before_last, Bar... bar) {
@@ -246,7 +277,7 @@ bool launch_coupled_rounds(Ctx& c, uint32_t steps, void (*kernel)(Args, const Ac
     const unsigned blocks = blocks_for(c.n, rounds * kCoupledBlock);
     const size_t smem = bytes * rounds * kCoupledBlock;
     constexpr size_t kFixed = 1024;  // at least the kernels' static shared memory
-    if (rounds * kCoupledBlock > 65536u || smem > (size_t)c.smem_optin - kFixed) {
+    if (!rounds_pay(c, steps, rounds, (uint64_t)slots * kCoupledBlock) || rounds * kCoupledBlock > 65536u || smem > (size_t)c.smem_optin - kFixed) {
         return false;
     }
     allow_shared_memory(c, kernel, kFixed);

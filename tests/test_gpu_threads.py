@@ -71,14 +71,14 @@ def test_blocks_of_small_and_large_networks(precision):
         rng = np.random.default_rng(n)
         net.set_positions(W.uniform_cube(n, (1000.0 * n) ** (1 / 3), 5), W.signal_types(n, 5))
         net.add_edges(rng.integers(0, n, n), rng.integers(0, n, n), np.ones(n, np.int32))
-        net.activity_block(1, 2)
+        net.activity_block(1, 3)
         net.synchronize()
         nets.append(net)
     before = [net.stats()["gpu_launches"] for net in nets]
 
     def loop(net):
         for k in range(6000):
-            net.activity_block(3 + 2 * k, 2)
+            net.activity_block(4 + 3 * k, 3)
         net.synchronize()
 
     failed = together(*(lambda net=net: loop(net) for net in nets))
