@@ -2003,13 +2003,17 @@ void launch_act32_h(Ctx& c, const ActVariant& v, const Act32& A, uint32_t kstep)
     }
 }
 
+constexpr uint32_t kPairsFrom = 250'000;
+
 template <int H, int MODEL = RL_MODEL_IZHIKEVICH>
 void launch_steps32(Ctx& c, const Act32& A, uint32_t nsteps, uint8_t* fired_before_last) {
     if constexpr (H > 0 && MODEL == RL_MODEL_IZHIKEVICH) {
-        // a batched context keeps a neuron per thread: in blocks of half its
-        // table's size the pairs are slower there (48 networks, 2.6M neurons:
-        // 13.6 us per step against 13.2)
-        if (!c.multi()) {
+        // a neuron per thread where pairs leave the device too few warps (us per
+        // step, single -> pairs: 20,000 neurons 0.69 -> 0.99, 100,000 1.13 ->
+        // 1.18, 200,000 1.72 -> 1.78, 300,000 2.29 -> 2.25, 1M 6.58 -> 6.26), and
+        // in a batched context: in blocks of half its table's size pairs are
+        // slower there (48 networks, 2.6M neurons: 13.2 -> 13.6)
+        if (!c.multi() && c.n >= kPairsFrom) {
             launch_pdl(&k_activity_f32_pairs<H, 128>, blocks_for((c.n + 1u) / 2u, 128), 128, c.stream, A, (const ActDesc*)c.act_desc.p, nsteps,
                        fired_before_last);
             return;
