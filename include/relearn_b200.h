@@ -386,8 +386,12 @@ RL_API rl_status rl_set_graphs(void* ctx, int enable);
  * simulation, before the first connections), a neuron's step reads nothing of
  * the other neurons, so a block of activity steps runs as one launch with each
  * neuron's state kept in registers for the whole block (1, the default); with
- * synapses, a network whose neurons all have a resident thread runs its blocks
- * in one launch too, with a device-wide barrier between steps.  0
+ * synapses, a network that fits the device (up to 1,136,640 neurons in FP64 and
+ * 1,875,456 in FP32) runs its blocks in one launch too, one or several neurons
+ * per thread and a device-wide barrier between steps, where that is faster: not
+ * with several networks in the context, and not with more than 113,664 (FP64) or
+ * 170,496 (FP32) neurons and very many synapses, or some of the AEIF and
+ * FitzHugh-Nagumo networks (act_coupled.cuh has the lines).  0
  * runs one launch per step.  The results are the same bits either way.  No
  * counterpart in the reference (its CPU loops run step by step). */
 RL_API rl_status rl_set_step_fusion(void* ctx, int enable);

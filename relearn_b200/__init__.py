@@ -595,7 +595,7 @@ class Network:
 
     def set_step_fusion(self, on: bool = True):
         """Blocks of activity steps of a network without synapses, or of one
-        with synapses whose neurons all have a resident thread, in one launch
+        with synapses that fits the device, in one launch where that is faster
         (the default), or one launch per step; the same bits."""
         self._check(self.lib.rl_set_step_fusion(self.h, int(on)))
 

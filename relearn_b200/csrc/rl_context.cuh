@@ -360,7 +360,7 @@ struct Ctx {
     uint32_t act_graph_len = 0;
     uint32_t act_block_len = 0;  // steps of the activity block being issued: only its last step stores the input
     bool use_graphs = true;
-    bool step_fusion = true;  // blocks of steps of a network without synapses in one launch
+    bool step_fusion = true;  // blocks of steps in one launch, without synapses or coupled (act_coupled.cuh)
     uint64_t fused_work = 0;  // neuron-steps of such a launch at most (0: the whole block)
     bool capturing = false;
     std::vector<NetInfo> nets;  // host copy

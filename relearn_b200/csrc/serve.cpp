@@ -243,8 +243,8 @@ struct Server {
         if ((st = rl_set_graphs(ctx, sc.use_graphs)) != RL_OK) {
             return fail(st, "rl_set_graphs");
         }
-        // Blocks of steps of a network without synapses in launches of at most
-        // kServeFusedWork neuron-steps: a whole block in one launch keeps its
+        // Blocks of steps in launches of at most kServeFusedWork neuron-steps
+        // (with synapses: a whole block of that size or one launch per step): a whole block in one launch keeps its
         // SMs for up to a millisecond and holds back the kernels of the
         // requests running beside it, one launch per step takes up to three
         // times as long.
