@@ -935,18 +935,29 @@ uint32_t wide_cap(const Ctx& c) {
     return (uint32_t)std::min<uint64_t>(kWideCap, (c.tree.num_nodes + 31) / 32 * 32);
 }
 
+// Warps of the ordered form for `open` searches: a full device's, in a serving
+// context no more than the scratch that a request's footprint (serve.cpp) has
+// room for: 8 MB and 96 B per neuron.
+uint32_t wide_slots(const Ctx& c, uint64_t open) {
+    uint64_t slots = std::min<uint64_t>(open, (uint64_t)c.num_sms * kWideWarpsPerSM);
+    if (c.fused_work) {
+        slots = std::min<uint64_t>(slots, (8'000'000 + 96ull * c.n) / (kWideEntryBytes * wide_cap(c)));
+    }
+    return (uint32_t)std::max<uint64_t>(slots, 1);
+}
+
 // The scratch of `slots` warps of `cap` entries each (grown as needed).
 WideSlot wide_scratch(Ctx& c, uint32_t slots, uint32_t cap) {
     Search& S = c.search;
     const size_t cells = (size_t)slots * cap;
-    S.w_node.ensure(cells);
-    S.w_info.ensure(cells);
-    S.w_child.ensure(cells);
-    S.w_cnt.ensure(cells);
-    S.w_pos.ensure(cells);
-    S.w_ord_node.ensure(cells);
-    S.w_w.ensure(cells);
-    S.w_ord_w.ensure(cells);
+    S.w_node.fit(cells);
+    S.w_info.fit(cells);
+    S.w_child.fit(cells);
+    S.w_cnt.fit(cells);
+    S.w_pos.fit(cells);
+    S.w_ord_node.fit(cells);
+    S.w_w.fit(cells);
+    S.w_ord_w.fit(cells);
     return WideSlot{ S.w_node.p, S.w_info.p, S.w_child.p, S.w_cnt.p, S.w_pos.p, S.w_ord_node.p, S.w_w.p, S.w_ord_w.p };
 }
 
@@ -1028,7 +1039,7 @@ void launch_wide(Ctx& c, const SearchArgs (&a)[2], const uint32_t (&warps)[2]) {
     if (!wide_redo_by_packets(c, open)) {
         constexpr int WPB = 4;
         const uint32_t cap = wide_cap(c);
-        const uint32_t slots = (uint32_t)std::min<uint64_t>(open, (uint64_t)c.num_sms * kWideWarpsPerSM);
+        const uint32_t slots = wide_slots(c, open);
         RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), st));
         WideArgs A;
         for (int t = 0; t < 2; ++t) {
@@ -1097,8 +1108,12 @@ SearchVariant default_search_shape(const Ctx& c, uint64_t m) {
 // searches in ten open, FP32 all), 20,000, 100,000 and 400,000 neurons
 // searching, ordered against packets: FP64 2.1, 13.6; 14.8, 26.2; 75, 58 ms;
 // FP32 3.7, 7.5; 28, 14.4; 148, 33 ms; 120,000 of 400,000 neurons searching:
-// FP64 23, 39; FP32 45, 23 ms.
+// FP64 23, 39; FP32 45, 23 ms.  Packets need no scratch, so they also take over
+// where a serving context has too few warps for the open searches.
 bool wide_redo_by_packets(const Ctx& c, uint64_t open) {
+    if (c.fused_work && open > 64ull * wide_slots(c, open)) {
+        return true;
+    }
     return open > (is_fp32(c) ? 60'000u : 250'000u) && 8 * open > c.search.num_searches;
 }
 

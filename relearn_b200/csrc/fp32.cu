@@ -2308,7 +2308,7 @@ void launch_search_wide_f32(Ctx& c, const uint32_t (&warps)[2], uint32_t segs0, 
     }
     if (!wide_redo_by_packets(c, open)) {
         const uint32_t cap = wide_cap(c);
-        const uint32_t slots = (uint32_t)std::min<uint64_t>(open, (uint64_t)c.num_sms * kWideWarpsPerSM);
+        const uint32_t slots = wide_slots(c, open);
         RL_CUDA_TRY(cudaMemsetAsync(S.tasks.p, 0, sizeof(uint32_t), c.stream));
         WideArgs32 W;
         for (int t = 0; t < 2; ++t) {

@@ -330,10 +330,12 @@ SearchVariant default_search_shape(const Ctx& c, uint64_t m);
 bool wide_redo_by_packets(const Ctx& c, uint64_t open);
 struct WideSlot;
 uint32_t wide_cap(const Ctx& c);
+uint32_t wide_slots(const Ctx& c, uint64_t open);
 WideSlot wide_scratch(Ctx& c, uint32_t slots, uint32_t cap);
 // one search per warp in the reference's order: walk entries per warp, warps per SM
 constexpr uint32_t kWideCap = 6144;
 constexpr uint32_t kWideWarpsPerSM = 16;
+constexpr uint32_t kWideEntryBytes = 40;  // of the eight arrays
 uint32_t hot_nodes(const Ctx& c, const SearchVariant& v, size_t node_bytes);
 const std::vector<ActVariant>& act_variants();
 
