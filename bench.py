@@ -218,42 +218,41 @@ CAPTURED = {
     # one launch per step at 1M neurons with synapses (bench.py --case
     # plasticity --step-fusion 0, launches of the second block): the step
     # kernel's DRAM read + write per launch plus that of a 64-step chunk's
-    # calcium and growth launch per step (FP64 34.95 + 0.11 MB + (97.04 +
-    # 7.33) / 64 MB; FP32 23.75 + 0.00 MB + (85.01 + 3.90) / 64 MB); FP64 warp
-    # instructions per neuron-step of both (DMUL, DADD, DFMA, DSETP: 6.26 +
-    # 3.72), and for the FP32 form warp instructions of every kind (7.98 +
-    # 1.36).  The FP64 pipe of an SM takes 2 warp instructions per cycle (64
-    # lanes).
-    "activity64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "e6ef1fe863ecbbd9",
-                   "traffic": 34.95e6 + 0.11e6 + (97.04e6 + 7.33e6) / 64, "fp64_warp_instr_per_neuron": 9.97},
-    "activity32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "ae16ba4013f08c25",
-                   "traffic": 23.75e6 + (85.01e6 + 3.90e6) / 64, "warp_instr_per_neuron": 9.34},
+    # calcium and growth launch per step; FP64 warp instructions per neuron-step
+    # of both (6.20 + 214.0 / 64), and for the FP32 form warp instructions of
+    # every kind (8.53 + 86.75 / 64).  The FP64 pipe of an SM takes 2 warp
+    # instructions per cycle (64 lanes).
+    "activity64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "7b41d7eb5ed5ecaa",
+                   "traffic": 26.14e6 + 0.01e6 + (97.05e6 + 7.41e6) / 64, "fp64_warp_instr_per_neuron": 9.54},
+    "activity32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "240ce99d557daa5c",
+                   "traffic": 15.13e6 + (85.02e6 + 3.32e6) / 64, "warp_instr_per_neuron": 9.89},
     # the fused block kernels (a network without synapses: a block of steps per
-    # launch, state in registers), from the instruction mix of one 100-step
-    # launch at 1M neurons (bench.py --case activity --case-steps 100), per
-    # neuron-step: k_activity_steps 9.05 warp instructions on the FP64 pipe;
-    # k_activity_f32_pairs 5.10 warp
-    # instructions of every kind, issued at one per SM sub-partition (4 per
-    # SM) per cycle; DRAM read + write of that launch
-    "fused64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "83fc480b4074af9a", "fp64_warp_instr_per_neuron": 9.05,
-                "traffic": 50.07e6 + 3.76e6},
-    "fused32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "66ca8356202a8dc8", "warp_instr_per_neuron": 5.10, "traffic": 30.02e6 + 0.19e6},
+    # launch, state in registers), from one 100-step launch at 1M neurons
+    # (bench.py --case activity --case-steps 100), per neuron-step:
+    # k_activity_steps 9.05 warp instructions on the FP64 pipe;
+    # k_activity_f32_pairs 4.98 warp instructions of every kind, issued at one
+    # per SM sub-partition (4 per SM) per cycle; DRAM read + write of that launch
+    "fused64": {"sources": ("activity.cu", "rl_math.cuh"), "digest": "7b41d7eb5ed5ecaa", "fp64_warp_instr_per_neuron": 9.05,
+                "traffic": 50.06e6 + 3.99e6},
+    "fused32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "240ce99d557daa5c", "warp_instr_per_neuron": 4.98, "traffic": 30.02e6 + 0.21e6},
     # the batched block kernel over the 128-network configuration (7.15M
     # neurons, bench.py --case ensemble --case-steps 100 --precision fp32):
     # warp instructions per neuron-step, DRAM read + write of the launch
-    "ensemble32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "ae16ba4013f08c25", "warp_instr_per_neuron": 5.95,
-                   "traffic": 215.10e6 + 187.94e6},
-    # a coupled block of 100 steps at 1M neurons with two synapses each, per
-    # neuron-step: FP32 warp instructions of every kind (k_activity_f32_coupled_rounds);
-    # FP64: the block kernel's, whose FP64 functions it runs
-    "coupled64": {"sources": ("act_coupled.cuh", "activity.cu", "rl_math.cuh"), "digest": "dfefc858881614f5", "fp64_warp_instr_per_neuron": 9.05},
-    "coupled32": {"sources": ("act_coupled.cuh", "fp32.cu", "rl_math.cuh"), "digest": "1c0a356d44151c38", "warp_instr_per_neuron": 9.58},
-    # the search snapshot at 1M (bench.py --case search; the excitatory pass,
-    # 0.8M searches): lanes active per warp instruction, L1 / L2 hit rates of
-    # the walk, DRAM bytes per search
-    "search64": {"sources": ("bh_search.cu", "bh_eval.cuh", "bh_wide.cuh", "rl_math.cuh"), "digest": "290d6ed0479e64d4", "lanes_active": 19.85,
-                 "l1_hit": 0.924, "l2_hit": 0.774, "dram_bytes_per_search": 681.0},
-    "search32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "ae16ba4013f08c25", "lanes_active": 21.88, "l1_hit": 0.812, "l2_hit": 0.936},
+    "ensemble32": {"sources": ("fp32.cu", "rl_math.cuh"), "digest": "240ce99d557daa5c", "warp_instr_per_neuron": 5.95,
+                   "traffic": 215.58e6 + 187.44e6},
+    # a coupled block of 100 steps at 1M neurons with a synapse each (the second
+    # block of bench.py --case plasticity), per neuron-step:
+    # k_activity_coupled_rounds' warp instructions on the FP64 pipe,
+    # k_activity_f32_coupled_rounds' of every kind
+    "coupled64": {"sources": ("act_coupled.cuh", "activity.cu", "rl_math.cuh"), "digest": "78166af43595b541", "fp64_warp_instr_per_neuron": 9.10},
+    "coupled32": {"sources": ("act_coupled.cuh", "fp32.cu", "rl_math.cuh"), "digest": "fa24c95c354cbc10", "warp_instr_per_neuron": 9.86},
+    # the search snapshot at 1M (bench.py --case search), one search per warp by
+    # bins: lanes active per warp instruction, L1 / L2 hit rates of the walk,
+    # DRAM bytes per search
+    "search64": {"sources": ("bh_bins.cuh", "bh_search.cu", "bh_eval.cuh", "rl_math.cuh"), "digest": "17efbf0a817a08a3", "lanes_active": 30.84,
+                 "l1_hit": 0.307, "l2_hit": 0.997, "dram_bytes_per_search": 268.5},
+    "search32": {"sources": ("bh_bins.cuh", "fp32.cu", "rl_math.cuh"), "digest": "0ab9f041e9a73939", "lanes_active": 31.65, "l1_hit": 0.431,
+                 "l2_hit": 0.996, "dram_bytes_per_search": 165.9},
 }
 B200_SMS = 148
 # algorithmic memory of a fused block launch per neuron: reads enabled, spike
@@ -327,6 +326,13 @@ def fused_roofline(precision: int, n: int, step_us: float, act_cnt: int, sm_mhz,
                  "hbm": {"bytes_per_launch": bytes_per_launch, "achieved": bytes_per_launch / (launch_us * 1e-6) / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": bytes_per_launch / (launch_us * 1e-6) / 1e9 / hbm if hbm else None, "peak_kind": peak_kind}})
     return roof
+
+
+def coupled_form(args, precision: int, n: int) -> str:
+    """The suffix of the kernel that runs a block of 100 steps of n Izhikevich
+    neurons with a few synapses each (act_coupled.cuh)."""
+    single, most = ((113_664, 1_136_640), (170_496, 1_875_456))[precision]
+    return "" if not args.step_fusion or n > most else ("_coupled" if n <= single else "_coupled_rounds")
 
 
 def step_compute(precision: int, n: int, step_us: float, sm_mhz=None, coupled: bool = False) -> dict:
@@ -665,17 +671,17 @@ def synapse_regime(args, dev, stream, world, precision):
     per_neuron = ACT_BYTES_PER_NEURON if precision == 0 else ACT_BYTES_FP32
     bytes_per_launch = step_bytes(precision, n, edges)
     act_achieved = bytes_per_launch / (act_ms / act_cnt / 1e3) / 1e9 if act_cnt else 0.0
-    act_roof = {"bound": "hbm", "kernel": ("k_activity" if precision == 0 else "k_activity_f32") + ("_coupled_rounds" if args.step_fusion else ""), "achieved": act_achieved, "peak": hbm,
+    act_roof = {"bound": "hbm", "kernel": ("k_activity" if precision == 0 else "k_activity_f32") + coupled_form(args, precision, n), "achieved": act_achieved, "peak": hbm,
                 "unit": "GB/s", "frac": act_achieved / hbm, "peak_kind": peak_kind, "bytes_per_launch": bytes_per_launch,
                 "avg_launch_us": 1e3 * act_ms / act_cnt if act_cnt else None, "launches": act_cnt,
                 "bytes": f"{per_neuron:.2f} B per neuron-step + {ACT_BYTES_PUSHED[precision]} B pushed sum per neuron-step + per 100-step block "
                          f"{ACT_BYTES_CSR_ROW} B row offsets per neuron and {ACT_BYTES_PER_EDGE} B per in-edge",
                 "kernels": "k_activity_coupled / k_activity_f32_coupled (_rounds): a block of steps in one launch, the state on chip between its steps; "
-                           "the bytes are those of one launch per step" if args.step_fusion else
+                           "the bytes are those of one launch per step" if coupled_form(args, precision, n) else
                            "the step kernel (k_activity / k_activity_f32, one launch per step) and the chunks' calcium and growth (k_calcium_growth / "
                            "k_calcium_growth_f32, one launch per chunk of up to 64 steps)"}
     if act_cnt:
-        comp = step_compute(precision, n, 1e3 * act_ms / act_cnt, coupled=bool(args.step_fusion))
+        comp = step_compute(precision, n, 1e3 * act_ms / act_cnt, coupled=bool(coupled_form(args, precision, n)))
         act_roof["compute"] = comp
         if comp["frac"] > act_roof["frac"]:
             # the arithmetic side is the nearer bound: report it first
@@ -696,7 +702,7 @@ def synapse_regime(args, dev, stream, world, precision):
         tps = touched / searches if precision == 0 else None
         out["bh_searches_per_s"] = searches / (search_ms / 1e3)
         if tps:
-            out["search_roofline"] = search_roofline(searches, tps, search_ms, precision)
+            out["search_roofline"] = search_roofline(searches, tps, search_ms, precision, net.tuning()["search_packet"])
     dom = max(("activity_kernel", "search_kernel", "connector", "graph", "commit", "tree_update"), key=lambda k: phases[k][0])
     out["dominant_phase"] = dom
     out["roofline"] = out.get("search_roofline") if dom == "search_kernel" and "search_roofline" in out else act_roof
@@ -938,20 +944,23 @@ def serve_figure(args, dev):
                          "bytes_per_neuron_step": per_ns}}
 
 
-def search_roofline(searches: float, touched_per_search: float, kernel_ms: float, precision: int) -> dict:
+def search_roofline(searches: float, touched_per_search: float, kernel_ms: float, precision: int, packet: int) -> dict:
     """The search against HBM by algorithmic bytes (acceptance tests the
     reference's walk runs x the node bytes of one test), with the bound that
     actually holds beside it: the walk is served from L1 / L2 (ncu DRAM bytes
-    per search are far below the algorithmic ones), so instruction issue with
-    idle lanes bounds it."""
+    per search are far below the algorithmic ones), so instruction issue and
+    the waits between its dependent loads bound it.  Lanes and hit rates are
+    those of one search per warp (packet 0)."""
     hbm, peak_kind = peaks()
     cap = captured("search64" if precision == 0 else "search32")
     bytes_per_search = touched_per_search * SEARCH_BYTES_PER_NODE
     achieved = searches * bytes_per_search / (kernel_ms * 1e-3) / 1e9
-    return {"bound": "issue (walk served from L1/L2)", "kernel": "k_search" if precision == 0 else "k_search_f32", "achieved": achieved,
+    kernel = ("k_search_bins", "k_search_bins32") if packet == 0 else ("k_search", "k_search_f32")
+    bins = packet == 0
+    return {"bound": "issue (walk served from L1/L2)", "kernel": kernel[precision], "achieved": achieved,
             "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind, "touched_per_search": touched_per_search,
-            "bytes_per_touched_node": SEARCH_BYTES_PER_NODE, "lanes_active_of_32": cap["lanes_active"], "l1_hit_rate": cap["l1_hit"],
-            "l2_hit_rate": cap["l2_hit"], "stale": cap["stale"],
+            "bytes_per_touched_node": SEARCH_BYTES_PER_NODE, "lanes_active_of_32": cap["lanes_active"] if bins else None,
+            "l1_hit_rate": cap["l1_hit"] if bins else None, "l2_hit_rate": cap["l2_hit"] if bins else None, "stale": cap["stale"] if bins else None,
             "how": "touched nodes from the library's counter (the acceptance tests the reference's walk runs) x bytes per node / search-kernel "
                    "time; lanes active and hit rates from ncu on the 1M snapshot"}
 
@@ -992,7 +1001,7 @@ def bh_snapshot(net, n, stream, step, precision=0, touched_per_search=None):
            "search_shape": {"warps_per_block": t["search_warps"], "packet": t["search_packet"], "register_cap": t["search_cap"], "hot_nodes": t["search_hot"],
                             "timed_ms": t["search_ms"]}}
     if touched_per_search:
-        out["roofline"] = search_roofline(searches, touched_per_search, min(search_ms), precision)
+        out["roofline"] = search_roofline(searches, touched_per_search, min(search_ms), precision, t["search_packet"])
         if precision == 1:
             out["roofline"]["touched_from"] = "the FP64 form's counter on the same snapshot (the same walk)"
     return out
